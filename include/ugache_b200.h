@@ -396,6 +396,10 @@ int ugc_refresh_commit(ugc_ctx* ctx);
  * (ids by descending count) gives the rank_ids / rank_freqs input of ugc_solve_placement. */
 int ugc_record(ugc_ctx* ctx, int replica_id, const void* keys, int key_bytes, size_t n, void* stream);
 int ugc_hotness_read(ugc_ctx* ctx, int replica_id, uint32_t* counts_out, int reset, void* stream);
+/* That ranking, on the host cores (host arrays of num_total_item entries; needs no GPU): rank_ids =
+ * ids by descending count, ties by ascending id; rank_freqs = their counts.  Replaces
+ * FreqRecorder::Sort (coll_cache_lib/freq_recorder.cc:207-274). */
+int ugc_rank_hotness(uint64_t num_total_item, const uint32_t* counts, uint32_t* rank_ids, uint32_t* rank_freqs);
 
 /* -- introspection --------------------------------------------------------------------- */
 int ugc_stats(ugc_ctx* ctx, int replica_id, ugc_stats_t* out);

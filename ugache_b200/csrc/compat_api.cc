@@ -18,7 +18,6 @@
 #include <map>
 #include <mutex>
 #include <numeric>
-#include <parallel/algorithm>
 #include <string>
 #include <thread>
 #include <vector>
@@ -265,15 +264,13 @@ int solve_to_shm(uint32_t epoch) {
     for (int64_t k = 0; k < (int64_t)N; k++) total[k] += f[k];
     if (mapped_here) munmap(f, N * 4);
   }
-  std::vector<uint32_t> ids(N);
-  std::iota(ids.begin(), ids.end(), 0u);
+  std::vector<uint32_t> ids(N), freqs(N);
   if (any) {
-    __gnu_parallel::stable_sort(ids.begin(), ids.end(),
-                                [&](uint32_t a, uint32_t b) { return total[a] > total[b]; });
+    int rc = ugc_rank_hotness(N, total.data(), ids.data(), freqs.data());
+    if (rc != UGC_OK) return pass(rc, "ugc_rank_hotness");
+  } else {
+    std::iota(ids.begin(), ids.end(), 0u);
   }
-  std::vector<uint32_t> freqs(N);
-#pragma omp parallel for
-  for (int64_t i = 0; i < (int64_t)N; i++) freqs[i] = total[ids[i]];
   void* base = shm_map(place_name(epoch), place_bytes(N, G), true);
   if (!base) return fail(UGC_ERR_NOMEM, "cannot create the placement segment in shared memory");
   PlaceView v = place_view(base, N, G);

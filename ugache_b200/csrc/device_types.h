@@ -167,8 +167,8 @@ __host__ __device__ inline uint32_t slot_pos(const SlotView& v, uint32_t j) {
 }
 
 // Classification of the whole id space into ascending key lists.
-//  build   (n2b_old == nullptr): list s = keys this reader fetches from GPU s, s in [0, G)
-//  refresh (n2b_old != nullptr): kListEvict  = stored here before, not now
+//  build   (src_old == nullptr): list s = keys this reader fetches from GPU s, s in [0, G)
+//  refresh (src_old != nullptr): kListEvict  = stored here before, not now
 //                                kListInsert = stored here now, not before
 //                                kListDropRemote = read from a peer before, source changed
 //                                kListAttach0+s  = read from peer s now, not before
@@ -180,17 +180,14 @@ constexpr int kMaxClassLists = kListAttach0 + kMaxDevice;  // 11
 struct RepointParams {
   TableView own;
   TableView peer[kMaxDevice];  // num_keys == 0: that peer's table is not known here
-  const uint32_t* n2b_new;     // device, N entries
-  const uint8_t* acc_new;      // device: this reader's source per block (new placement)
+  const uint8_t* src_new;      // device, N entries: this reader's source per key (new placement)
   uint32_t me;
   uint32_t num_device;
 };
 
 struct ClassifyParams {
-  const uint32_t* n2b_old;   // device, N entries, or nullptr
-  const uint32_t* n2b_new;   // device, N entries
-  const uint8_t* acc_old;    // device: this reader's source per block (old placement)
-  const uint8_t* acc_new;    // device: same for the new placement
+  const uint8_t* src_old;    // device, N entries: this reader's source per key, or nullptr
+  const uint8_t* src_new;    // device, N entries: same for the new placement
   uint64_t num_keys;
   uint32_t me;
   uint32_t num_device;

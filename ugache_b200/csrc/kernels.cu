@@ -1267,7 +1267,7 @@ __global__ void __launch_bounds__(kBlock)
   bool ok = false;
   if (key < t.num_keys) {
     uint32_t word_new = kEmptyWord;
-    const uint32_t src_new = p.acc_new[p.n2b_new[key]];
+    const uint32_t src_new = p.src_new[key];
     if (src_new < p.num_device && src_new != p.me && p.peer[src_new].num_keys) {
       const uint32_t w = table_lookup(p.peer[src_new], key);
       if (w != kEmptyWord && word_loc(w) == src_new) word_new = w;
@@ -1374,9 +1374,9 @@ constexpr int kClassRounds = kClassTile / kBlock;
 
 // Bit mask of the lists key k belongs to (see ClassifyParams in device_types.h).
 __device__ __forceinline__ uint32_t class_mask(const ClassifyParams& p, uint64_t k) {
-  const uint32_t src_new = p.acc_new[p.n2b_new[k]];
-  if (p.n2b_old == nullptr) return src_new < p.num_device ? (1u << src_new) : 0u;  // build
-  const uint32_t src_old = p.acc_old[p.n2b_old[k]];
+  const uint32_t src_new = p.src_new[k];
+  if (p.src_old == nullptr) return src_new < p.num_device ? (1u << src_new) : 0u;  // build
+  const uint32_t src_old = p.src_old[k];
   if (src_old == src_new) return 0u;
   uint32_t m = 0;
   if (src_old == p.me) m |= 1u << kListEvict;

@@ -90,11 +90,17 @@ LinkDesc b200_link_desc(int num_device, uint32_t row_bytes, double bw_local_over
 // plus UGC_POLICY_SPLIT_SEARCH, which has no counterpart among them: it stands in for the
 // reference's MILP (optimal_solver_class.cc:957-1112) on a switch-connected box by costing every
 // replicate/partition split against the recorded hotness.
-// cache_percent in percent.  Returns an empty string or the reason for failure.
+// cache_percent in percent.  Returns an empty string or the reason for failure.  The per-key array
+// goes to `nid_to_block` (N entries of the caller's) if that is given, else into *out.
 std::string solve_placement(int policy, int num_device, uint64_t num_total_item,
                             const uint32_t* rank_ids, const uint32_t* rank_freqs,
                             double cache_percent, double t_local, double t_remote, double t_cpu,
-                            Placement* out);
+                            Placement* out, uint32_t* nid_to_block = nullptr);
+
+// Ids by descending count, ties by ascending id, and the counts in that order (replaces
+// FreqRecorder::Sort, coll_cache_lib/freq_recorder.cc:207-274).  Returns false when the host has
+// no memory for the pass buffer (8 bytes per id, given back before the call returns).
+bool rank_hotness(uint64_t num_total_item, const uint32_t* counts, uint32_t* rank_ids, uint32_t* rank_freqs);
 
 // Modelled cost of a placement per reader under the concurrent-source model the split-search
 // policy minimises: max((local + served to peers + 1) * t_local, peers * t_remote, host * t_cpu),

@@ -324,6 +324,11 @@ class Cache:
     @staticmethod
     def rank_hotness(counts):
         """(rank_ids, rank_freqs) for the placement solvers: ids by descending count, ties by id."""
+        if counts.dtype == np.uint32 and counts.ndim == 1:  # what hotness_read returns
+            counts = np.ascontiguousarray(counts)
+            ids, freqs = np.empty(len(counts), np.uint32), np.empty(len(counts), np.uint32)
+            check(_lib.lib().ugc_rank_hotness(len(counts), _ptr(counts), _ptr(ids), _ptr(freqs)))
+            return ids, freqs
         order = np.argsort(-counts.astype(np.int64), kind="stable").astype(np.uint32)
         return order, counts[order]
 
