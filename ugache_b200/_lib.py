@@ -7,6 +7,7 @@ import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libugache_b200.so")
+FAST_PATH = os.path.join(HERE, "_fast.so")
 
 UGC_MAX_DEVICE = 8
 UGC_OK = 0
@@ -214,6 +215,29 @@ def lib():
                               "expected %s): rebuild with `python -m ugache_b200.build`"
                               % (list(sizes), mine))
     return _lib
+
+
+_fast = None
+
+
+def fast():
+    """The extension module with the per-step calls (needs torch); raises if it has not been built."""
+    global _fast
+    if _fast is None:
+        import importlib.util
+
+        import torch  # noqa: F401  (its libraries have to be in the process first)
+        if not os.path.exists(FAST_PATH):
+            raise ImportError("_fast.so is missing (%s): build it with `python -m ugache_b200.build`" % FAST_PATH)
+        L = lib()
+        spec = importlib.util.spec_from_file_location("ugache_b200._fast", FAST_PATH)
+        m = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(m)
+        m.bind(check, {name: C.cast(getattr(L, name), C.c_void_p).value
+                       for name in ("ugc_lookup_i64", "ugc_lookup_u32", "ugc_lookup_unique", "ugc_lookup_pool",
+                                    "ugc_record")})
+        _fast = m
+    return _fast
 
 
 def check(status):

@@ -1,7 +1,7 @@
 """Python face of the C ABI: a thin object wrapper that moves pointers, nothing else.
 
 PyTorch appears here only to own device memory and streams; every operation is a call
-into ``libugache_b200.so``.
+into ``libugache_b200.so``, the per-step ones through the extension module ``_fast.so``.
 """
 import ctypes as C
 
@@ -14,6 +14,8 @@ from ._lib import (POLICY_CLIQUE_PART, POLICY_INTUITIVE, POLICY_REP, POLICY_SPLI
 POLICIES = {"intuitive": POLICY_INTUITIVE, "coll_intuitive": POLICY_INTUITIVE,
             "rep": POLICY_REP, "clique_part": POLICY_CLIQUE_PART,
             "split_search": POLICY_SPLIT_SEARCH}
+_ELEM = {"f32": 0, "f16": 1}
+_POOL_MODE = {"sum": 0, "mean": 1}
 
 
 class PlacementArrays:
@@ -125,6 +127,8 @@ class Cache:
         self.cfg = cfg
         self._h = C.c_void_p()
         check(L.ugc_create(C.byref(cfg), C.byref(self._h)))
+        self._ctx = self._h.value  # what the extension module takes
+        self._row_bytes = row_bytes
         self._keep = []  # host arrays the library reads in place
 
     # -- lifetime -----------------------------------------------------------------
@@ -132,6 +136,7 @@ class Cache:
         if self._h:
             _lib.lib().ugc_destroy(self._h)
             self._h = C.c_void_p()
+            self._ctx = 0
 
     def __del__(self):
         try:
@@ -188,40 +193,16 @@ class Cache:
     def lookup(self, replica_id, keys, out=None, stream=None):
         """keys: CUDA tensor (int64 / int32 / uint32); returns a uint8 [n, row_bytes] tensor
         unless ``out`` (any dtype, n*row_bytes bytes) is given."""
-        import torch
-        n = keys.numel()
-        if keys.dtype == torch.int64:
-            kb = 8
-        elif keys.dtype in (torch.int32, torch.uint32):
-            kb = 4
-        else:
-            raise TypeError("keys must be int64, int32 or uint32")
-        if out is None:
-            out = torch.empty((n, self.cfg.row_bytes), dtype=torch.uint8, device=keys.device)
-        s = torch.cuda.current_stream(keys.device).cuda_stream if stream is None else stream
-        self.lookup_ptr(replica_id, keys.data_ptr(), kb, n, out.data_ptr(), s)
-        return out
+        return (_lib._fast or _lib.fast()).lookup(self._ctx, replica_id, self._row_bytes, keys, out, stream)
 
     def lookup_unique(self, replica_id, keys, stream=None):
         """Deduplicated lookup on the GPU.  keys: CUDA tensor (int64 / int32).  Returns
         ``(rows, unique_keys, inverse, n_unique)``: uint8 ``rows[n, row_bytes]`` of which the
         first ``n_unique`` are filled, ``unique_keys[n]`` likewise, int32 ``inverse[n]`` and a
         one-element int32 tensor ``n_unique`` -- all on the device, nothing synchronises."""
-        import torch
-        keys = keys.reshape(-1)
-        n = keys.numel()
-        kb = 8 if keys.dtype == torch.int64 else 4
-        dev = keys.device
-        rows = torch.empty((n, self.cfg.row_bytes), dtype=torch.uint8, device=dev)
-        uniq = torch.empty_like(keys)
-        inverse = torch.empty(n, dtype=torch.int32, device=dev)
-        n_unique = torch.zeros(1, dtype=torch.int32, device=dev)
-        s = torch.cuda.current_stream(dev).cuda_stream if stream is None else stream
-        check(_lib.lib().ugc_lookup_unique(self._h, replica_id, C.c_void_p(keys.data_ptr()), kb, n,
-                                           C.c_void_p(rows.data_ptr()), C.c_void_p(uniq.data_ptr()),
-                                           C.c_void_p(inverse.data_ptr()), C.c_void_p(n_unique.data_ptr()),
-                                           C.c_void_p(s)))
-        return rows, uniq, inverse, n_unique
+        if keys.dim() != 1:
+            keys = keys.reshape(-1)
+        return (_lib._fast or _lib.fast()).lookup_unique(self._ctx, replica_id, self._row_bytes, keys, stream)
 
     def lookup_pool(self, replica_id, keys, offsets=None, bag_size=0, elem="f32", mode="sum", out=None,
                     stream=None):
@@ -229,30 +210,22 @@ class Cache:
         added in key order.  keys: CUDA tensor (int64 / int32); offsets: CUDA int64 tensor of
         ``n_bags + 1`` positions, or None with ``bag_size`` keys per bag.  Returns the
         ``[n_bags, dim]`` fp32 tensor."""
-        import torch
-        keys = keys.reshape(-1)
-        n = keys.numel()
-        kb = 8 if keys.dtype == torch.int64 else 4
-        dev = keys.device
+        if keys.dim() != 1:
+            keys = keys.reshape(-1)
         if offsets is not None:
+            import torch
             if offsets.dtype != torch.int64 or not offsets.is_cuda:
                 raise ValueError("offsets must be a CUDA int64 tensor")
             offsets = offsets.contiguous()
-            n_bags = offsets.numel() - 1
+            n_bags = max(offsets.numel() - 1, 0)
         else:
             if bag_size <= 0:
                 raise ValueError("give offsets or a bag size")
-            n_bags = n // bag_size
-        elem_type = {"f32": 0, "f16": 1}[elem]
-        dim = self.cfg.row_bytes // (2 if elem_type else 4)
-        if out is None:
-            out = torch.empty((max(n_bags, 0), dim), dtype=torch.float32, device=dev)
-        s = torch.cuda.current_stream(dev).cuda_stream if stream is None else stream
-        check(_lib.lib().ugc_lookup_pool(self._h, replica_id, C.c_void_p(keys.data_ptr()), kb, n,
-                                         C.c_void_p(offsets.data_ptr() if offsets is not None else None),
-                                         max(n_bags, 0), bag_size, elem_type, {"sum": 0, "mean": 1}[mode],
-                                         C.c_void_p(out.data_ptr()), C.c_void_p(s)))
-        return out
+            n_bags = keys.numel() // bag_size
+        elem_type = _ELEM[elem]
+        return (_lib._fast or _lib.fast()).lookup_pool(
+            self._ctx, replica_id, keys, offsets, n_bags, bag_size, elem_type, _POOL_MODE[mode],
+            self._row_bytes // (2 if elem_type else 4), out, stream)
 
     def lookup_pool_ptr(self, replica_id, keys_ptr, key_bytes, n_keys, offsets_ptr, n_bags, bag_size,
                         elem_type, mode, out_ptr, stream=0):
@@ -309,11 +282,7 @@ class Cache:
     # -- hotness ---------------------------------------------------------------------------
     def record(self, replica_id, keys, stream=None):
         """Count the accesses of a CUDA key tensor (int64 / int32) on the device."""
-        import torch
-        kb = 8 if keys.dtype == torch.int64 else 4
-        s = torch.cuda.current_stream(keys.device).cuda_stream if stream is None else stream
-        check(_lib.lib().ugc_record(self._h, replica_id, C.c_void_p(keys.data_ptr()), kb,
-                                    keys.numel(), C.c_void_p(s)))
+        (_lib._fast or _lib.fast()).record(self._ctx, replica_id, keys, stream)
 
     def hotness_read(self, replica_id, reset=False, stream=0):
         counts = np.empty(self.cfg.num_total_item, dtype=np.uint32)
