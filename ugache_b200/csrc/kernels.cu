@@ -1494,15 +1494,52 @@ __global__ void __launch_bounds__(kBlock)
 // ------------------------------------------------------------------------------------
 // hotness recording: per-key access counts of a batch, kept on the device
 // ------------------------------------------------------------------------------------
+// What bounds it is the L2's rate of additions to ONE address (0.6 ns each): the hottest id is 18 %
+// of a Zipf-1.2 batch, 38,000 additions of 212,992, which took 22 us one by one.  So the hot ids are
+// added up before they leave the SM: lanes of a warp that hold the same id find each other (match)
+// and count once, and a direct-mapped set of kRecordSlots counters in shared memory, one per id
+// that comes first, takes the warps' counts; an id whose slot is taken goes straight to the L2.
+// 1024 keys a CTA: enough for the hot ids to meet, few enough to fill the SMs from 150 k keys on.
+constexpr int kRecordKpt = 4;
+constexpr uint32_t kRecordSlots = 1024;
+
 template <typename KeyT>
 __global__ void __launch_bounds__(kBlock)
     record_kernel(const KeyT* __restrict__ keys, uint32_t n, uint32_t* __restrict__ counts,
                   uint64_t num_keys) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint64_t k = (uint64_t)keys[i];
-  if (k < num_keys) atomicAdd(counts + k, 1u);  // fire-and-forget reduction in L2
+  __shared__ uint32_t s_key[kRecordSlots], s_cnt[kRecordSlots];
+  const uint32_t base = blockIdx.x * (kBlock * kRecordKpt) + threadIdx.x;
+  uint32_t key[kRecordKpt];
+#pragma unroll
+  for (int j = 0; j < kRecordKpt; j++) {
+    const uint64_t i = (uint64_t)base + j * kBlock;
+    const uint64_t k = i < n ? (uint64_t)keys[i] : num_keys;
+    key[j] = k < num_keys ? (uint32_t)k : kEmptyWord;  // also drops negative int64 ids
+  }
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  for (uint32_t i = threadIdx.x; i < kRecordSlots; i += kBlock) {
+    s_key[i] = kEmptyWord;
+    s_cnt[i] = 0;
+  }
+  __syncthreads();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < kRecordKpt; j++) {
+    const unsigned same = __match_any_sync(kFull, key[j]);
+    if (key[j] == kEmptyWord || (threadIdx.x & 31) != (uint32_t)(__ffs(same) - 1)) continue;
+    const uint32_t slot = (key[j] * 2654435761u) >> 22;
+    const uint32_t held = atomicCAS(&s_key[slot], kEmptyWord, key[j]);
+    if (held == kEmptyWord || held == key[j]) {
+      atomicAdd(&s_cnt[slot], (uint32_t)__popc(same));
+    } else {
+      atomicAdd(counts + key[j], (uint32_t)__popc(same));  // fire-and-forget reduction in L2
+    }
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < kRecordSlots; i += kBlock)
+    if (s_cnt[i]) atomicAdd(counts + s_key[i], s_cnt[i]);
 }
+static_assert(kRecordSlots == 1u << 10, "the slot is the top 10 bits of the hash");
 
 // ------------------------------------------------------------------------------------
 // synthetic table rows
@@ -1925,14 +1962,12 @@ cudaError_t launch_classify_scatter(const ClassifyParams& p, const void* scratch
 cudaError_t launch_record(const void* keys, int key_bytes, uint32_t n, uint32_t* counts,
                           uint64_t num_keys, cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
-  if (key_bytes == 8) {
-    record_kernel<long long><<<grid_for(n), kBlock, 0, stream>>>(static_cast<const long long*>(keys), n,
-                                                                counts, num_keys);
-  } else {
-    record_kernel<uint32_t><<<grid_for(n), kBlock, 0, stream>>>(static_cast<const uint32_t*>(keys), n,
-                                                               counts, num_keys);
-  }
-  return cudaGetLastError();
+  const int grid = (int)(((uint64_t)n + kBlock * kRecordKpt - 1) / (kBlock * kRecordKpt));
+  if (key_bytes == 8)
+    return launch_pdl(record_kernel<long long>, grid, kBlock, 0, stream, true,
+                      static_cast<const long long*>(keys), n, counts, num_keys);
+  return launch_pdl(record_kernel<uint32_t>, grid, kBlock, 0, stream, true,
+                    static_cast<const uint32_t*>(keys), n, counts, num_keys);
 }
 
 cudaError_t launch_gen_table(void* dst, uint64_t seed, uint64_t row_begin, uint64_t n_rows,
