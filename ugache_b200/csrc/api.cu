@@ -1057,7 +1057,6 @@ int do_lookup(ugc_ctx* c, Replica* r, const void* keys, int key_bytes, size_t n,
     // counts of the direct launch before it
     d.slot = r->direct_slot;
     d.publish_prev = r->last_was_direct ? 1u : 0u;
-    d.prev_keys = r->last_n;
     d.prev_seq = r->last_seq;
     r->direct_slot ^= 1u;
     r->last_slot = d.slot;

@@ -75,16 +75,16 @@ struct Counters {
   // launch adds to its slot and clears the other one (whose launch is complete by then)
   uint32_t dcount[2][kNumGroup];
   uint32_t reserved3[2];
+  alignas(16) uint32_t shown[kNumGroup + 1];  // what the pinned mirror shows: counts and ordinal
   // pooled lookups: rows summed so far, per source group (cumulative)
   unsigned long long pool_rows[kNumGroup];
 };
 
-// Written by the last CTA of every extraction into pinned host memory: the host reads it
+// Written by an extraction into pinned host memory when its counts have moved: the host reads it
 // without synchronising to pick the extraction mode of the lookups it enqueues next.
-struct Feedback {
-  uint32_t keys;
+struct alignas(16) Feedback {
   uint32_t count[kNumGroup];
-  uint32_t seq;  // ordinal of the lookup these counts belong to (written last; 0 = none yet)
+  uint32_t seq;  // ordinal of the lookup these counts belong to (0 = none yet)
 };
 
 // Everything the role-partitioned gather needs.
@@ -149,7 +149,6 @@ struct DirectParams {
   uint32_t tile_shift;  // log2 of the keys one warp probes at a time (3..5)
   uint32_t slot;        // which of Counters::dcount this launch adds to (launches alternate)
   uint32_t publish_prev;  // 1: the launch before this one was a direct one; hand its counts on
-  uint32_t prev_keys;     // its batch size
   uint32_t prev_seq;      // its ordinal among the replica's lookups
 };
 
