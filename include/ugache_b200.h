@@ -413,12 +413,13 @@ typedef struct {
   uint32_t struct_size;
   int32_t gather_ctas_per_sm;     /* CTAs of the gather kernel per SM                       */
   int32_t gather_block_threads;   /* 256, 512 or 1024                                       */
-  int32_t gather_vec_bytes;       /* 16 or 32 bytes per lane per load                       */
-  int32_t host_ctas;              /* most CTAs the host-row group may take                       */
+  int32_t gather_vec_bytes;       /* 16 or 32 bytes per lane per load of the gather         */
+  int32_t host_ctas;              /* most CTAs the host-row group may take (left at its default: fewer
+                                     for a host list in address order and rows below 1 KB)   */
   int32_t remote_ctas;            /* most CTAs the peer-row group may take                       */
   int32_t bulk_mask;              /* far sources staged through shared memory by the
                                      bulk-async copy engine: bit 0 host rows, bit 1 peer rows */
-  int32_t lookup_keys_per_thread; /* 1, 2 or 4                                              */
+  int32_t lookup_keys_per_thread; /* 1, 2 or 4; 0 (default) = chosen by the batch size       */
   int32_t programmatic_launch;    /* programmatic stream serialization: bit 0 for the lookup
                                      kernel (its key loads and probes overlap the tail of
                                      the previous gather), bit 1 for the gather kernel (it is
@@ -437,8 +438,8 @@ typedef struct {
                                      it, so that the host link's queue stays filled from one
                                      lookup to the next: 0 = when the last finished lookup took
                                      at least 1024 host rows, 1 = always, 2 = never          */
-  int32_t host_order_min_rows;    /* grouped extraction: order the host list by address (two
-                                     small kernels between lookup and gather) when the last
+  int32_t host_order_min_rows;    /* grouped extraction: order the host list by address (one
+                                     small kernel between lookup and gather) when the last
                                      finished lookup took at least this many rows from the
                                      host table; 0 = never                                  */
   int32_t refresh_fill_ctas;      /* refresh-time fill: CTAs per launch (20, as the reference,

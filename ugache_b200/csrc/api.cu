@@ -504,15 +504,22 @@ struct DevBuf {
 };
 
 // Pinned, GPU-mapped host memory of one replica: the mirror the lookups write their counts to, and
-// what the build and refresh steps stage.
-constexpr uint64_t kStageKeys = 1u << 19;
-constexpr int kStageParts = 4;
-struct PinnedStage {
+// what the build and refresh steps read back.
+struct PinnedBlock {
   Feedback feedback;
   unsigned long long totals[kMaxClassLists];
   unsigned long long err_table;
-  uint8_t src[kStageParts][kStageKeys];
 };
+
+// Pinned staging between pageable host arrays and the GPU: one block of kStageParts parts for the
+// whole process, taken by one build / refresh / hotness step at a time, which leaves no copy in
+// flight behind.  Made on first use (2-3 ms: per cache it would be a third of a small build) and
+// given back with the last context.
+constexpr uint64_t kStageKeys = 1u << 19;
+constexpr int kStageParts = 4;
+std::mutex g_stage_mu;
+uint8_t* g_stage = nullptr;
+int g_contexts = 0;
 
 struct Replica {
   bool built = false;
@@ -536,7 +543,10 @@ struct Replica {
   void* ipc_opened[2 * kMaxDevice] = {nullptr};
   int n_ipc_opened = 0;
   // lookup scratch
+  DevBuf scratch;  // one block: range counts of the host list, the lists, the ordered host list
   uint64_t* list[kNumGroup] = {nullptr, nullptr, nullptr};
+  uint64_t* host_sorted = nullptr;  // host list in address order
+  uint32_t* host_hist = nullptr;    // its range counts: zero between lookups
   Counters* counters = nullptr;
   uint32_t max_batch = 0;
   // host-buffer lookups
@@ -567,8 +577,6 @@ struct Replica {
   std::vector<cudaEvent_t> copy_events;
   uint32_t* stamp = nullptr;               // deduplicated lookups: one stamp per id (first use)
   uint32_t stamp_epoch = 0;
-  uint64_t* host_sorted = nullptr;         // host list in address order (allocated on first use)
-  uint32_t* host_hist = nullptr;
   int host_order_min_rows = 8192;
   uint64_t lookups_host_ordered = 0;
   uint32_t direct_slot = 0, last_slot = 0; // count slot of the next / the last direct launch
@@ -577,7 +585,7 @@ struct Replica {
   cudaStream_t recent_streams[4] = {nullptr, nullptr, nullptr, nullptr};  // streams lookups ran on
   bool recent_valid[4] = {false, false, false, false};
   int direct_block = 256;
-  int direct_max_host_rows = 8192;
+  int direct_max_host_rows = 4096;
   int direct_tile_shift = 0;               // 0: chosen per launch
   int direct_deep = 0;
   int direct_early_host = 0;               // 0 auto, 1 always, 2 never
@@ -587,8 +595,8 @@ struct Replica {
   // classification (build: one list per source; refresh: evict / insert / drop / attach).
   uint8_t* src_dev = nullptr;              // this reader's source per key, current placement
   uint8_t* src_next = nullptr;             // same for the placement a refresh is moving to
-  PinnedStage* pinned = nullptr;
-  cudaEvent_t pinned_ev[kStageParts] = {};
+  PinnedBlock* pinned = nullptr;
+  cudaEvent_t stage_ev[kStageParts] = {};
   DevBuf class_scratch;
   DevBuf lists;                            // all lists back to back
   uint64_t list_count[kMaxClassLists] = {0};
@@ -599,10 +607,11 @@ struct Replica {
   uint64_t lookups = 0;
   int gather_grid = 0;
   int host_ctas = 0, remote_ctas = 0;
+  int host_ctas_default = 0;  // host_ctas as the link description gave it
   int vec_bytes = 32;
   int block_threads = 256;
   int bulk_mask = 0;
-  int lookup_kpt = 1;
+  int lookup_kpt = 0;  // 0: chosen per launch
   int pdl = 3;  // bit 0: lookup kernel, bit 1: gather kernel launched with programmatic serialization
   // extraction mode: UGC_EXTRACT_AUTO / _GROUPED / _DIRECT; in auto mode the choice follows
   // the host-row share of the last finished lookup, read from the pinned mirror below
@@ -631,7 +640,6 @@ struct ugc_ctx {
   bool host_registered_here = false;
   size_t host_registered_bytes = 0;
   std::mutex mu;
-  std::mutex stage_mu;  // the replicas' pinned staging parts
   // device memory held now: through the caller's allocator / obtained by the library itself
   // (cudaMalloc or virtual-memory blocks), for ugc_stats
   std::mutex acct_mu;
@@ -856,16 +864,25 @@ void release_lists(ugc_ctx* c, Replica* r) {
 int make_pinned(Replica* r) {
   void* p = nullptr;
   void* dev = nullptr;
-  UGC_CUDA(cudaHostAlloc(&p, sizeof(PinnedStage), cudaHostAllocMapped));
-  r->pinned = static_cast<PinnedStage*>(p);
-  for (auto& e : r->pinned_ev) UGC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  UGC_CUDA(cudaHostAlloc(&p, sizeof(PinnedBlock), cudaHostAllocMapped));
+  r->pinned = static_cast<PinnedBlock*>(p);
+  for (auto& e : r->stage_ev) UGC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   memset(&r->pinned->feedback, 0, sizeof(Feedback));
   if (cudaHostGetDevicePointer(&dev, p, 0) == cudaSuccess) {
     r->feedback = &r->pinned->feedback;
-    r->feedback_dev = &static_cast<PinnedStage*>(dev)->feedback;
+    r->feedback_dev = &static_cast<PinnedBlock*>(dev)->feedback;
   } else {  // without the mirror the auto mode stays on the grouped path
     cudaGetLastError();
   }
+  return UGC_OK;
+}
+
+// The process' staging block; g_stage_mu held.
+int make_stage() {
+  if (g_stage) return UGC_OK;
+  void* p = nullptr;
+  UGC_CUDA(cudaHostAlloc(&p, kStageParts * kStageKeys, cudaHostAllocPortable));
+  g_stage = static_cast<uint8_t*>(p);
   return UGC_OK;
 }
 
@@ -882,18 +899,20 @@ int upload_sources(ugc_ctx* c, Replica* r, const Placement& p, uint8_t** dst, cu
   const uint8_t* acc = &p.block_access_from[(size_t)r->id * p.num_block];
   const uint32_t* n2b = p.nid_to_block.data();
   const int threads = std::max(1, std::min(16, omp_get_num_procs()));
-  std::lock_guard<std::mutex> lock(c->stage_mu);
+  std::lock_guard<std::mutex> lock(g_stage_mu);
+  UGC_TRY(make_stage());
   int buf = 0;
   for (uint64_t off = 0; off < N; off += kStageKeys, buf = (buf + 1) % kStageParts) {
     const int64_t m = (int64_t)std::min<uint64_t>(kStageKeys, N - off);
-    uint8_t* stage = r->pinned->src[buf];
-    UGC_CUDA(cudaEventSynchronize(r->pinned_ev[buf]));  // the copy that used this part before
+    uint8_t* stage = g_stage + buf * kStageKeys;
+    UGC_CUDA(cudaEventSynchronize(r->stage_ev[buf]));  // the copy that used this part before
     const uint32_t* from = n2b + off;
 #pragma omp parallel for schedule(static) num_threads(m > 65536 ? threads : 1)
     for (int64_t i = 0; i < m; i++) stage[i] = acc[from[i]];
     UGC_CUDA(cudaMemcpyAsync(*dst + off, stage, (size_t)m, cudaMemcpyHostToDevice, s));
-    UGC_CUDA(cudaEventRecord(r->pinned_ev[buf], s));
+    UGC_CUDA(cudaEventRecord(r->stage_ev[buf], s));
   }
+  for (auto& e : r->stage_ev) UGC_CUDA(cudaEventSynchronize(e));
   return UGC_OK;
 }
 
@@ -911,11 +930,9 @@ void release_replica(ugc_ctx* c, Replica* r) {
     if (!dev_block_free(r->ipc_opened[i])) cudaIpcCloseMemHandle(r->ipc_opened[i]);
   ctx_free_shared(c, r->slice);
   ctx_free_shared(c, r->table_mem);
-  for (auto& l : r->list) ctx_free(c, l);
+  ctx_free(c, r->scratch.ptr);
   ctx_free(c, r->counters);
   ctx_free(c, r->free_ring);
-  ctx_free(c, r->host_sorted);
-  ctx_free(c, r->host_hist);
   ctx_free(c, r->stamp);
   ctx_free(c, r->hot_counts);
   ctx_free(c, r->src_dev);
@@ -927,9 +944,29 @@ void release_replica(ugc_ctx* c, Replica* r) {
   ctx_free(c, r->stage_a.ptr);
   ctx_free(c, r->stage_b.ptr);
   if (r->pinned) cudaFreeHost(r->pinned);
-  for (cudaEvent_t e : r->pinned_ev)
+  for (cudaEvent_t e : r->stage_ev)
     if (e) cudaEventDestroy(e);
   *r = Replica{};
+}
+
+// Lookup scratch for batches of up to max_batch keys, as one block.
+int make_scratch(ugc_ctx* c, DevBuf* out, uint32_t max_batch, cudaStream_t s) {
+  const size_t list = round_up((size_t)max_batch * sizeof(uint64_t), 256);
+  const size_t bytes = host_order_scratch_bytes() + (kNumGroup + 1) * list;
+  out->ptr = ctx_alloc(c, bytes);
+  if (!out->ptr) return fail(UGC_ERR_NOMEM, "scratch allocation for %u keys failed", max_batch);
+  out->bytes = bytes;
+  UGC_CUDA(cudaMemsetAsync(out->ptr, 0, host_order_scratch_bytes(), s));
+  return UGC_OK;
+}
+void use_scratch(Replica* r, uint32_t max_batch) {
+  char* p = static_cast<char*>(r->scratch.ptr);
+  r->host_hist = reinterpret_cast<uint32_t*>(p);
+  p += host_order_scratch_bytes();
+  const size_t list = round_up((size_t)max_batch * sizeof(uint64_t), 256);
+  for (int g = 0; g < kNumGroup; g++, p += list) r->list[g] = reinterpret_cast<uint64_t*>(p);
+  r->host_sorted = reinterpret_cast<uint64_t*>(p);
+  r->max_batch = max_batch;
 }
 
 GatherParams gather_params(ugc_ctx* c, Replica* r, void* out, uint32_t n) {
@@ -1068,7 +1105,7 @@ int do_lookup(ugc_ctx* c, Replica* r, const void* keys, int key_bytes, size_t n,
       const volatile Feedback* f = r->feedback;
       early = f->seq != 0 && f->count[kGroupHost] >= 1024u;
     }
-    UGC_CUDA(launch_extract_direct(keys, key_bytes, d, r->direct_grid, r->direct_block, r->vec_bytes, r->direct_deep != 0,
+    UGC_CUDA(launch_extract_direct(keys, key_bytes, d, r->direct_grid, r->direct_block, r->direct_deep != 0,
                                    early && d.host_base != nullptr, (r->pdl & 1) != 0 && n_dev == nullptr, s));
     if (prof) {
       UGC_CUDA(cudaEventRecord(r->prof_events[r->prof_used + 2], s));
@@ -1082,25 +1119,27 @@ int do_lookup(ugc_ctx* c, Replica* r, const void* keys, int key_bytes, size_t n,
     remember_stream(r, s);
     return UGC_OK;
   }
+  // many host rows last time: this lookup's host list is put in address order before the gather
+  uint32_t* hist = want_host_order(r) ? r->host_hist : nullptr;
+  const uint64_t host_rows = c->cfg.empty_feat > 0 ? ((uint64_t)1 << c->cfg.empty_feat) : c->cfg.num_total_item;
   UGC_CUDA(launch_lookup_group(keys, key_bytes, (uint32_t)n, r->table, (uint32_t)r->id,
                                (uint32_t)c->cfg.num_device, c->cfg.empty_feat, r->list[kGroupLocal],
-                               r->list[kGroupRemote], r->list[kGroupHost], r->counters, r->lookup_kpt, (r->pdl & 1) != 0, s));
+                               r->list[kGroupRemote], r->list[kGroupHost], r->counters, r->lookup_kpt, hist, host_rows,
+                               (r->pdl & 1) != 0, s));
   if (prof) UGC_CUDA(cudaEventRecord(r->prof_events[r->prof_used + 1], s));
   GatherParams p = gather_params(c, r, out, (uint32_t)n);
-  if (want_host_order(r)) {
-    // many host rows last time: order this lookup's host list by address before the gather
-    if (!r->host_sorted) {
-      r->host_sorted = static_cast<uint64_t*>(ctx_alloc(c, (size_t)r->max_batch * sizeof(uint64_t)));
-      r->host_hist = static_cast<uint32_t*>(ctx_alloc(c, host_order_scratch_bytes()));
-    }
-    if (r->host_sorted && r->host_hist) {
-      const uint64_t host_rows = c->cfg.empty_feat > 0 ? ((uint64_t)1 << c->cfg.empty_feat) : c->cfg.num_total_item;
-      UGC_CUDA(launch_host_order(r->list[kGroupHost], r->host_sorted, r->counters, r->host_hist, host_rows,
-                                 r->sm_count, s));
-      p.list[kGroupHost] = r->host_sorted;
-      r->kernel_launches += 2;
-      r->lookups_host_ordered++;
-    }
+  if (hist) {
+    UGC_CUDA(launch_host_order(r->list[kGroupHost], r->host_sorted, r->counters, hist, host_rows, r->sm_count,
+                               (r->pdl & 2) != 0, s));
+    p.list[kGroupHost] = r->host_sorted;
+    p.host_hist = hist;
+    // CTAs for an ordered list: 40 keep 2560 rows of 256 bytes in flight, which is the window the
+    // order pays for (128- and 256-byte rows over 32 GB: 14.2 and 23.4 GB/s, with 148 CTAs 11.4 and
+    // 20.3); rows of 512 bytes fill the link from 80 CTAs on (46.9 GB/s with 40, 49.3 with 80)
+    if (r->host_ctas == r->host_ctas_default)
+      p.host_cta_cap = std::min(r->host_ctas, 40 * (int)std::max(1u, c->cfg.row_bytes / 256));
+    r->kernel_launches += 1;
+    r->lookups_host_ordered++;
   }
   UGC_CUDA(launch_gather_roles(p, r->gather_grid, r->block_threads, r->vec_bytes, s));
   if (prof) {
@@ -1226,6 +1265,10 @@ int ugc_create(const ugc_config* cfg, ugc_ctx** out) {
   if (!c) return fail(UGC_ERR_NOMEM, "out of host memory");
   c->cfg = *cfg;
   c->reps.resize(cfg->num_device);
+  {
+    std::lock_guard<std::mutex> lock(g_stage_mu);
+    g_contexts++;
+  }
   *out = c;
   return UGC_OK;
 }
@@ -1236,6 +1279,13 @@ int ugc_destroy(ugc_ctx* c) {
     if (r.built) release_replica(c, &r);
   if (c->host_registered_here && c->host_table)
     ugc_host_unregister_sized(const_cast<void*>(c->host_table), c->host_registered_bytes);
+  {
+    std::lock_guard<std::mutex> lock(g_stage_mu);
+    if (--g_contexts == 0 && g_stage) {
+      cudaFreeHost(g_stage);
+      g_stage = nullptr;
+    }
+  }
   delete c;
   return UGC_OK;
 }
@@ -1418,14 +1468,17 @@ int ugc_build(ugc_ctx* c, int replica_id, int device_id, const void* host_table,
     const LinkDesc ld = b200_link_desc(G, c->cfg.row_bytes, c->cfg.bw_local_gbs, c->cfg.bw_remote_gbs,
                                        c->cfg.bw_host_gbs);
     r->host_ctas = c->cfg.host_ctas > 0 ? c->cfg.host_ctas : ld.host_ctas;
+    r->host_ctas_default = c->cfg.host_ctas > 0 ? 0 : ld.host_ctas;
     r->remote_ctas = c->cfg.remote_ctas > 0 ? c->cfg.remote_ctas : ld.remote_ctas;
     r->t_byte[kGroupLocal] = (float)(1.0 / ld.bw_local_gbs);
     r->t_byte[kGroupRemote] = ld.bw_remote_gbs > 0 ? (float)(1.0 / ld.bw_remote_gbs) : 0.0f;
     r->t_byte[kGroupHost] = (float)(1.0 / ld.bw_host_gbs);
   }
-  // 32-byte loads win when almost every row comes from HBM (8 GPUs, 458 host rows per batch:
-  // 36.5 us per step against 45); with more host rows per batch 16-byte loads were faster
-  // (1 GPU: 113 vs 133 us, 2 GPUs: 84 vs 110 us, 4 GPUs: 54 vs 61 us).
+  // Loads of the gather: 32 bytes win when almost every row comes from HBM (8 GPUs, 458 host rows
+  // per batch: 36.5 us per step against 45); with more host rows per batch 16-byte loads were faster
+  // (1 GPU: 113 vs 133 us, 2 GPUs: 84 vs 110 us, 4 GPUs: 54 vs 61 us).  The direct kernel takes the
+  // widest the addresses allow (90.0 against 93.5 us with 7,277 host rows per batch, 2.4 against 2.6
+  // for 208 keys, equal without host rows).
   r->vec_bytes = c->cfg.gather_vec_bytes ? (c->cfg.gather_vec_bytes == 32 ? 32 : 16) : (G >= 8 ? 32 : 16);
 
   // 1. which source serves each key: ascending key lists per GPU source, made on the GPU
@@ -1470,11 +1523,8 @@ int ugc_build(ugc_ctx* c, int replica_id, int device_id, const void* host_table,
   };
   int rc;
   // 3. lookup scratch and counters
-  r->max_batch = c->cfg.max_batch;
-  for (int g = 0; g < kNumGroup; g++) {
-    r->list[g] = static_cast<uint64_t*>(ctx_alloc(c, (size_t)r->max_batch * sizeof(uint64_t)));
-    if (!r->list[g]) return bail(fail(UGC_ERR_NOMEM, "scratch allocation failed"));
-  }
+  if ((rc = make_scratch(c, &r->scratch, c->cfg.max_batch, s)) != UGC_OK) return bail(rc);
+  use_scratch(r, c->cfg.max_batch);
   r->counters = static_cast<Counters*>(ctx_alloc(c, sizeof(Counters)));
   if (!r->counters) return bail(fail(UGC_ERR_NOMEM, "counter allocation failed"));
   if (cudaMemsetAsync(r->counters, 0, sizeof(Counters), s) != cudaSuccess)
@@ -1729,7 +1779,7 @@ int ugc_lookup_i64_static(ugc_ctx* c, int replica_id, const int64_t* keys, size_
   UGC_CUDA(cudaMemsetAsync(counters, 0, sizeof(Counters), s));
   UGC_CUDA(launch_lookup_group(keys, 8, (uint32_t)n, r->table, (uint32_t)r->id, (uint32_t)c->cfg.num_device,
                                c->cfg.empty_feat, lists, lists + kStaticMaxKeys, lists + 2 * (size_t)kStaticMaxKeys,
-                               counters, r->lookup_kpt, false, s));
+                               counters, r->lookup_kpt, nullptr, 0, false, s));
   GatherParams p{};
   for (int i = 0; i < kMaxLocation; i++) p.src_base[i] = r->src_base[i];
   p.out = out;
@@ -1836,21 +1886,19 @@ int ugc_reserve_batch(ugc_ctx* c, int replica_id, uint32_t max_batch) {
   if (max_batch <= r->max_batch) return UGC_OK;
   UGC_CUDA(cudaSetDevice(r->device));
   UGC_TRY(drain_lookups(r));  // the old lists may still be in use by lookups in flight
-  uint64_t* fresh[kNumGroup] = {nullptr, nullptr, nullptr};
-  for (int g = 0; g < kNumGroup; g++) {
-    fresh[g] = static_cast<uint64_t*>(ctx_alloc(c, (size_t)max_batch * sizeof(uint64_t)));
-    if (!fresh[g]) {
-      for (int k = 0; k < g; k++) ctx_free(c, fresh[k]);
-      return fail(UGC_ERR_NOMEM, "scratch allocation for %u keys failed", max_batch);
-    }
+  DevBuf fresh;
+  int rc = make_scratch(c, &fresh, max_batch, nullptr);
+  if (rc == UGC_OK && cudaStreamSynchronize(nullptr) != cudaSuccess)
+    rc = fail(UGC_ERR_CUDA, "scratch set-up failed: %s", cudaGetErrorString(cudaGetLastError()));
+  if (rc != UGC_OK) {
+    std::string keep = g_last_error;
+    ctx_free(c, fresh.ptr);
+    g_last_error = keep;
+    return rc;
   }
-  for (int g = 0; g < kNumGroup; g++) {
-    ctx_free(c, r->list[g]);
-    r->list[g] = fresh[g];
-  }
-  ctx_free(c, r->host_sorted);  // sized by max_batch: re-made on the next ordered lookup
-  r->host_sorted = nullptr;
-  r->max_batch = max_batch;
+  ctx_free(c, r->scratch.ptr);
+  r->scratch = fresh;
+  use_scratch(r, max_batch);
   return UGC_OK;
 }
 
@@ -2124,7 +2172,8 @@ int ugc_hotness_read(ugc_ctx* c, int replica_id, uint32_t* counts_out, int reset
   // The caller's array is pageable: the counters come through the parts of the pinned staging
   // block, up to three crossing PCIe while the host threads copy the oldest out (8 MB: 450-680 us
   // through the driver's own staging, which copies with one thread).
-  std::lock_guard<std::mutex> lock(c->stage_mu);
+  std::lock_guard<std::mutex> lock(g_stage_mu);
+  UGC_TRY(make_stage());
   const int threads = std::max(1, std::min(16, omp_get_num_procs()));
   const size_t pieces = (bytes + kStageKeys - 1) / kStageKeys;
   auto length = [&](size_t i) { return std::min<size_t>(kStageKeys, bytes - i * kStageKeys); };
@@ -2132,15 +2181,14 @@ int ugc_hotness_read(ugc_ctx* c, int replica_id, uint32_t* counts_out, int reset
   for (size_t i = 0; i < pieces; i++) {
     for (; sent < pieces && sent < i + kStageParts; sent++) {
       const int buf = (int)(sent % kStageParts);
-      UGC_CUDA(cudaEventSynchronize(r->pinned_ev[buf]));  // an upload that used this part before
-      UGC_CUDA(cudaMemcpyAsync(r->pinned->src[buf], reinterpret_cast<const char*>(r->hot_counts) + sent * kStageKeys,
+      UGC_CUDA(cudaMemcpyAsync(g_stage + buf * kStageKeys, reinterpret_cast<const char*>(r->hot_counts) + sent * kStageKeys,
                                length(sent), cudaMemcpyDeviceToHost, s));
-      UGC_CUDA(cudaEventRecord(r->pinned_ev[buf], s));
+      UGC_CUDA(cudaEventRecord(r->stage_ev[buf], s));
     }
     const int64_t len = (int64_t)length(i);
-    const uint8_t* from = r->pinned->src[i % kStageParts];
+    const uint8_t* from = g_stage + (i % kStageParts) * kStageKeys;
     char* to = reinterpret_cast<char*>(counts_out) + i * kStageKeys;
-    UGC_CUDA(cudaEventSynchronize(r->pinned_ev[i % kStageParts]));
+    UGC_CUDA(cudaEventSynchronize(r->stage_ev[i % kStageParts]));
 #pragma omp parallel for schedule(static) num_threads(len > 65536 ? threads : 1)
     for (int64_t at = 0; at < len; at += 16384) memcpy(to + at, from + at, (size_t)std::min<int64_t>(16384, len - at));
   }
@@ -2239,7 +2287,7 @@ int ugc_set_tuning(ugc_ctx* c, int replica_id, const ugc_tuning* t) {
   const int bt = t->gather_block_threads, kpt = t->lookup_keys_per_thread, vec = t->gather_vec_bytes;
   if (t->gather_ctas_per_sm < 1 || t->gather_ctas_per_sm > 32 || (bt != 256 && bt != 512 && bt != 1024) ||
       (vec != 16 && vec != 32) || t->host_ctas < 1 || t->remote_ctas < 1 || t->bulk_mask < 0 ||
-      t->bulk_mask > 3 || (kpt != 1 && kpt != 2 && kpt != 4) || t->extract_mode < UGC_EXTRACT_AUTO ||
+      t->bulk_mask > 3 || (kpt != 0 && kpt != 1 && kpt != 2 && kpt != 4) || t->extract_mode < UGC_EXTRACT_AUTO ||
       t->extract_mode > UGC_EXTRACT_DIRECT || t->direct_ctas_per_sm < 1 || t->direct_ctas_per_sm > 16 ||
       t->direct_max_host_rows < 0 || (t->direct_block_threads != 128 && t->direct_block_threads != 256) ||
       t->host_zero_copy < 0 || t->host_zero_copy > 3)

@@ -94,6 +94,7 @@ struct GatherParams {
   const uint64_t* list[kNumGroup];
   Counters* counters;
   Feedback* feedback;   // pinned host mirror of the last lookup's counts, or nullptr
+  uint32_t* host_hist;  // the host list is in address order: its range counts, to be cleared; or nullptr
   uint32_t row_bytes;
   uint32_t n_keys;
   int remote_cta_cap;   // most CTAs of the peer group: what keeps the NVLink port full

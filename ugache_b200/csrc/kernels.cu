@@ -164,15 +164,24 @@ __device__ __forceinline__ uint32_t table_lookup(const TableView& t, uint32_t ke
   return probe_rest(t.slots, t.line_mask, key, line);
 }
 
+// Address range of a host row, for the ordering of the host list.
+constexpr int kHostBuckets = 4096;
+__device__ __forceinline__ uint32_t host_bucket(uint32_t off, uint32_t shift) {
+  return min(off >> shift, (uint32_t)kHostBuckets - 1);
+}
+
 // ------------------------------------------------------------------------------------
 // lookup + group by source
 // ------------------------------------------------------------------------------------
+// What bounds it is latency and, with one key per thread, the three list counters, which sit in one
+// sector of the L2 and take one addition every 0.6 ns: 6,656 CTAs x 3 of them were half of the 38 us
+// a batch of 1.7 M keys took.  Four keys a thread make a quarter of the CTAs.
 template <typename KeyT, int kKeysPerThread>
 __global__ void __launch_bounds__(kBlock)
     lookup_group_kernel(const KeyT* __restrict__ keys, uint32_t n, TableView t, uint32_t local_loc,
                         uint32_t host_loc, uint32_t host_mask, uint64_t* __restrict__ list_local,
                         uint64_t* __restrict__ list_remote, uint64_t* __restrict__ list_host,
-                        Counters* counters) {
+                        Counters* counters, uint32_t* host_hist, uint32_t hist_shift) {
   __shared__ uint32_t s_cnt[kWarpsPerBlock][kKeysPerThread][kNumGroup];
   __shared__ uint32_t s_base[kNumGroup];
 
@@ -256,6 +265,9 @@ __global__ void __launch_bounds__(kBlock)
       group[j] = (loc == local_loc) ? kGroupLocal : kGroupRemote;
     }
     if (!valid[j]) group[j] = kNumGroup;
+    // address range of a host row, counted for the ordering of the host list (below)
+    if (host_hist != nullptr && group[j] == (uint32_t)kGroupHost)
+      atomicAdd(&host_hist[host_bucket(off, hist_shift)], 1u);
     rec[j] = make_record(idx, loc, off);
     rank_in_warp[j] = 0;
 #pragma unroll
@@ -379,6 +391,9 @@ __device__ __forceinline__ void split_roles(const GatherParams& p, const uint32_
     return max(n, 1);
   };
   n_host = share(t_host, cnt[kGroupHost], p.host_cta_cap);
+  // an ordered host list is worked by a set number of CTAs: with more, the rows in flight spread
+  // over more of the table than the order is worth
+  if (p.host_hist && cnt[kGroupHost]) n_host = max(1, min(p.host_cta_cap, ceil_div_i(cnt[kGroupHost], rmin)));
   n_remote = share(t_rem, cnt[kGroupRemote], p.remote_cta_cap);
   if (p.fixed_split) {
     n_host = cnt[kGroupHost] ? max(p.host_cta_cap, 1) : 0;
@@ -538,6 +553,11 @@ __global__ void __launch_bounds__(1024) gather_roles_kernel(GatherParams p) {
   int n_host, n_remote;
   split_roles(p, cnt, grid, n_host, n_remote);
 
+  // the counts behind the host list's order are used up: zero again for the next lookup
+  if (p.host_hist && b == grid - 1)
+    for (uint32_t i = threadIdx.x; i < 2 * kHostBuckets / 4; i += blockDim.x)
+      reinterpret_cast<uint4*>(p.host_hist)[i] = make_uint4(0, 0, 0, 0);
+
   const uint32_t vecs_per_row = p.row_bytes / VEC;
   const uint32_t workers_per_cta = blockDim.x / LPR;
   const uint32_t worker_in_cta = threadIdx.x / LPR;
@@ -611,6 +631,7 @@ __global__ void __launch_bounds__(1024) gather_roles_kernel(GatherParams p) {
       const uint32_t total =
           gg == kGroupLocal ? cnt[kGroupLocal] : (gg == kGroupRemote ? cnt[kGroupRemote] : cnt[kGroupHost]);
       if (total == 0) continue;
+      if (k > 0 && gg == kGroupHost && p.host_hist) continue;  // ordered: see split_roles
       const int ctas_gg = gg == kGroupLocal ? grid - n_host - n_remote : (gg == kGroupRemote ? n_remote : n_host);
       const uint32_t owned = (uint32_t)ctas_gg * chunk;  // rows covered by the first chunks
       if (k > 0 && owned >= total) continue;             // nothing beyond them to take
@@ -731,51 +752,56 @@ __global__ void __launch_bounds__(kBlock)
 // ------------------------------------------------------------------------------------
 // host list in address order
 // ------------------------------------------------------------------------------------
-// Scattered rows of pinned host memory arrive about 15 % faster when the reads in flight move
-// through the table in ascending address order (63-68 M against 55-60 M rows per second,
-// measured with nothing else running), which is what the reference gets from sorting its
-// whole index (coll_cache_lib/cache_context.cu:702-761).  Here only the host list is ordered,
-// and only coarsely: a counting sort into kHostBuckets address ranges.  Two small kernels
-// between the lookup and the gather; `hist` holds kHostBuckets counts followed by
-// kHostBuckets cursors, all zero on entry.
-constexpr int kHostBuckets = 256;
+// Rows of pinned host memory arrive faster when the reads in flight lie close together and move
+// through the table in ascending order, which is what the reference gets from sorting its whole
+// index (coll_cache_lib/cache_context.cu:702-761).  Measured with nothing else running, random
+// against ordered (kHostBuckets ranges): 128-byte rows 37 -> 49 GB/s over a 1 GB table and 8.9 ->
+// 14.2 over 32 GB, 256-byte rows 17.7 -> 23.4 over 32 GB, 512-byte rows 35.7 -> 38.0.  256 ranges
+// gave a third of that over 32 GB: the window of rows in flight has to be narrower than a range.
+// Only the host list is ordered, by a counting sort: the lookup counts the ranges while it emits the
+// list, one small kernel scatters it, the gather clears the counts for the next lookup.
+// `hist` holds kHostBuckets counts followed by kHostBuckets cursors, all zero on entry.
+constexpr int kScatterBlock = 512;
+constexpr int kBucketsPerThread = kHostBuckets / kScatterBlock;
 
-__device__ __forceinline__ uint32_t host_bucket(uint64_t rec, uint32_t shift) {
-  const uint32_t b = rec_off(rec) >> shift;
-  return b < (uint32_t)kHostBuckets ? b : (uint32_t)kHostBuckets - 1;
-}
-
-__global__ void __launch_bounds__(kBlock)
-    host_hist_kernel(const uint64_t* __restrict__ list, const Counters* counters, uint32_t* hist,
-                     uint32_t shift) {
-  __shared__ uint32_t s_hist[kHostBuckets];
-  for (int i = threadIdx.x; i < kHostBuckets; i += kBlock) s_hist[i] = 0;
-  __syncthreads();
-  const uint32_t n = counters->count[kGroupHost];
-  for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock)
-    atomicAdd(&s_hist[host_bucket(list[i], shift)], 1u);
-  __syncthreads();
-  for (int i = threadIdx.x; i < kHostBuckets; i += kBlock)
-    if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
-}
-
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kScatterBlock)
     host_scatter_kernel(const uint64_t* __restrict__ list, uint64_t* __restrict__ sorted,
                         const Counters* counters, uint32_t* hist, uint32_t shift) {
   __shared__ uint32_t s_start[kHostBuckets];
-  if (threadIdx.x == 0) {  // exclusive prefix of the bucket counts (256 adds, same in every CTA)
-    uint32_t run = 0;
-    for (int i = 0; i < kHostBuckets; i++) {
-      s_start[i] = run;
-      run += hist[i];
-    }
+  __shared__ uint32_t s_warp[kScatterBlock / 32];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // exclusive prefix of the counts, the same in every CTA
+  uint32_t cnt[kBucketsPerThread], sum = 0;
+  const uint4* h4 = reinterpret_cast<const uint4*>(hist) + threadIdx.x * (kBucketsPerThread / 4);
+#pragma unroll
+  for (int i = 0; i < kBucketsPerThread / 4; i++) {
+    const uint4 h = __ldcg(h4 + i);
+    cnt[4 * i] = h.x, cnt[4 * i + 1] = h.y, cnt[4 * i + 2] = h.z, cnt[4 * i + 3] = h.w;
+    sum += h.x + h.y + h.z + h.w;
+  }
+  uint32_t x = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t y = __shfl_up_sync(kFull, x, d);
+    if (lane >= (uint32_t)d) x += y;
+  }
+  if (lane == 31) s_warp[warp] = x;
+  __syncthreads();
+  uint32_t run = x - sum;
+  for (uint32_t w = 0; w < warp; w++) run += s_warp[w];
+#pragma unroll
+  for (int i = 0; i < kBucketsPerThread; i++) {
+    s_start[threadIdx.x * kBucketsPerThread + i] = run;
+    run += cnt[i];
   }
   __syncthreads();
   uint32_t* cursor = hist + kHostBuckets;
   const uint32_t n = counters->count[kGroupHost];
-  for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
+  for (uint32_t i = blockIdx.x * kScatterBlock + threadIdx.x; i < n; i += gridDim.x * kScatterBlock) {
     const uint64_t rec = list[i];
-    const uint32_t b = host_bucket(rec, shift);
+    const uint32_t b = host_bucket(rec_off(rec), shift);
     sorted[s_start[b] + atomicAdd(&cursor[b], 1u)] = rec;
   }
 }
@@ -1682,6 +1708,13 @@ inline uint32_t host_mask_of(int empty_feat) {
   return empty_feat > 0 && empty_feat < 32 ? ((1u << empty_feat) - 1u) : 0xffffffffu;
 }
 
+// bucket = row offset >> shift: kHostBuckets ranges over the host table
+inline uint32_t host_order_shift(uint64_t host_rows) {
+  uint32_t shift = 0;
+  while (shift < 31 && (host_rows >> shift) > (uint64_t)kHostBuckets) shift++;
+  return shift;
+}
+
 }  // namespace
 
 // ------------------------------------------------------------------------------------
@@ -1690,14 +1723,17 @@ inline uint32_t host_mask_of(int empty_feat) {
 cudaError_t launch_lookup_group(const void* keys, int key_bytes, uint32_t n, const TableView& table,
                                 uint32_t local_loc, uint32_t host_loc, int empty_feat,
                                 uint64_t* list_local, uint64_t* list_remote, uint64_t* list_host,
-                                Counters* counters, int keys_per_thread, bool pdl,
-                                cudaStream_t stream) {
+                                Counters* counters, int keys_per_thread, uint32_t* host_hist,
+                                uint64_t host_rows, bool pdl, cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
   const uint32_t mask = host_mask_of(empty_feat);
+  const uint32_t shift = host_order_shift(host_rows);
+  // 0: four keys a thread once that still leaves every SM four CTAs, one below
+  if (keys_per_thread == 0) keys_per_thread = n >= 148u * 4 * kBlock * 4 ? 4 : 1;
 #define UGC_LAUNCH_LOOKUP(KEYT, KPT)                                                             \
   return launch_pdl(lookup_group_kernel<KEYT, KPT>, (int)((n + kBlock * KPT - 1) / (kBlock * KPT)), \
                     kBlock, 0, stream, pdl, static_cast<const KEYT*>(keys), n, table, local_loc,   \
-                    host_loc, mask, list_local, list_remote, list_host, counters)
+                    host_loc, mask, list_local, list_remote, list_host, counters, host_hist, shift)
   if (key_bytes == 8) {
     if (keys_per_thread == 1) UGC_LAUNCH_LOOKUP(long long, 1);
     if (keys_per_thread == 2) UGC_LAUNCH_LOOKUP(long long, 2);
@@ -1720,13 +1756,12 @@ int usable_vec_bytes(uint32_t row_bytes, int want, const void* out, const void* 
 }
 
 cudaError_t launch_extract_direct(const void* keys, int key_bytes, const DirectParams& p_in, int grid,
-                                  int block, int vec_bytes, bool deep, bool early_host, bool pdl,
-                                  cudaStream_t stream) {
+                                  int block, bool deep, bool early_host, bool pdl, cudaStream_t stream) {
   if (block != 128 && block != 256) block = kBlock;
   const int warps_per_block = block / 32;
   if (p_in.n_keys == 0) return cudaSuccess;
   DirectParams p = p_in;
-  const int vec = usable_vec_bytes(p.row_bytes, vec_bytes, p.out, p.src_base, kMaxLocation);
+  const int vec = usable_vec_bytes(p.row_bytes, 32, p.out, p.src_base, kMaxLocation);
   const int lpr = lanes_per_row(p.row_bytes, vec);
   p.lpr_shift = 0;
   while ((1 << p.lpr_shift) < lpr) p.lpr_shift++;
@@ -1859,14 +1894,9 @@ cudaError_t launch_unique(const void* keys, int key_bytes, uint32_t n, uint64_t 
 size_t host_order_scratch_bytes() { return 2 * kHostBuckets * sizeof(uint32_t); }
 
 cudaError_t launch_host_order(const uint64_t* list_host, uint64_t* sorted, const Counters* counters,
-                              uint32_t* hist, uint64_t host_rows, int sm_count, cudaStream_t stream) {
-  cudaError_t e = cudaMemsetAsync(hist, 0, host_order_scratch_bytes(), stream);
-  if (e != cudaSuccess) return e;
-  uint32_t shift = 0;  // bucket = row offset >> shift, kHostBuckets buckets over the host table
-  while (shift < 32 && (host_rows >> shift) > (uint64_t)kHostBuckets) shift++;
-  host_hist_kernel<<<sm_count, kBlock, 0, stream>>>(list_host, counters, hist, shift);
-  host_scatter_kernel<<<sm_count, kBlock, 0, stream>>>(list_host, sorted, counters, hist, shift);
-  return cudaGetLastError();
+                              uint32_t* hist, uint64_t host_rows, int sm_count, bool pdl, cudaStream_t stream) {
+  return launch_pdl(host_scatter_kernel, sm_count, kScatterBlock, 0, stream, pdl, list_host, sorted, counters, hist,
+                    host_order_shift(host_rows));
 }
 
 cudaError_t launch_gather_roles(const GatherParams& p_in, int grid, int block, int vec_bytes,

@@ -20,11 +20,15 @@ namespace ugc {
 
 // All launchers enqueue on `stream` and return the launch status; none synchronises.
 
+// keys_per_thread: 1, 2 or 4; 0 = chosen by the batch size.  host_hist: nullptr, or the scratch of
+// launch_host_order (host_order_scratch_bytes(), zero on entry), in which the host rows of the
+// batch are counted per address range of the `host_rows` rows.
+
 cudaError_t launch_lookup_group(const void* keys, int key_bytes, uint32_t n, const TableView& table,
                                 uint32_t local_loc, uint32_t host_loc, int empty_feat,
                                 uint64_t* list_local, uint64_t* list_remote, uint64_t* list_host,
-                                Counters* counters, int keys_per_thread, bool pdl,
-                                cudaStream_t stream);
+                                Counters* counters, int keys_per_thread, uint32_t* host_hist,
+                                uint64_t host_rows, bool pdl, cudaStream_t stream);
 
 cudaError_t launch_gather_roles(const GatherParams& p, int grid, int block, int vec_bytes,
                                 cudaStream_t stream);
@@ -44,12 +48,12 @@ cudaError_t launch_unique(const void* keys, int key_bytes, uint32_t n, uint64_t 
 cudaError_t launch_lookup_pool(const void* keys, int key_bytes, const PoolParams& p, bool f16,
                                int max_ctas, int vec_bytes, cudaStream_t stream);
 
-// Orders the host list of the lookup just enqueued by address range (counting sort into 256
-// buckets over `host_rows` rows) into `sorted`; `hist` is host_order_scratch_bytes() of scratch.
-// Enqueue between launch_lookup_group and launch_gather_roles and hand `sorted` to the gather.
+// Orders the host list of the lookup just enqueued by address range into `sorted`; `hist` as handed
+// to launch_lookup_group.  Enqueue between launch_lookup_group and launch_gather_roles, hand
+// `sorted` to the gather as its host list and `hist` as GatherParams::host_hist.
 size_t host_order_scratch_bytes();
 cudaError_t launch_host_order(const uint64_t* list_host, uint64_t* sorted, const Counters* counters,
-                              uint32_t* hist, uint64_t host_rows, int sm_count, cudaStream_t stream);
+                              uint32_t* hist, uint64_t host_rows, int sm_count, bool pdl, cudaStream_t stream);
 
 // Lookup and row copy in one kernel (no index lists): out[i] = row of keys[i].  `grid` is
 // the most CTAs to use (a multiple of the SM count); fewer are launched for small batches.
@@ -58,8 +62,7 @@ cudaError_t launch_host_order(const uint64_t* list_host, uint64_t* sorted, const
 // `early_host` (ignored with `deep`): the first host row of every warp's first tile is fetched
 // before the kernel waits for the launch ahead of it.
 cudaError_t launch_extract_direct(const void* keys, int key_bytes, const DirectParams& p, int grid,
-                                  int block, int vec_bytes, bool deep, bool early_host, bool pdl,
-                                  cudaStream_t stream);
+                                  int block, bool deep, bool early_host, bool pdl, cudaStream_t stream);
 
 // Widest of 32 / 16 / 4 bytes, not above `want`, that divides row_bytes and the address of
 // `out` and of every non-null source base: rows then start on a multiple of it on both sides.
