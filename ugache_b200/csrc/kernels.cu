@@ -1560,6 +1560,13 @@ __global__ void __launch_bounds__(kBlock)
     record_kernel(const KeyT* __restrict__ keys, uint32_t n, uint32_t* __restrict__ counts,
                   uint64_t num_keys) {
   __shared__ uint32_t s_key[kRecordSlots], s_cnt[kRecordSlots];
+  for (uint32_t i = threadIdx.x; i < kRecordSlots; i += kBlock) {
+    s_key[i] = kEmptyWord;
+    s_cnt[i] = 0;
+  }
+  // the keys are read behind the dependency wait: they may be what the launch ahead writes
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t base = blockIdx.x * (kBlock * kRecordKpt) + threadIdx.x;
   uint32_t key[kRecordKpt];
 #pragma unroll
@@ -1568,13 +1575,7 @@ __global__ void __launch_bounds__(kBlock)
     const uint64_t k = i < n ? (uint64_t)keys[i] : num_keys;
     key[j] = k < num_keys ? (uint32_t)k : kEmptyWord;  // also drops negative int64 ids
   }
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  for (uint32_t i = threadIdx.x; i < kRecordSlots; i += kBlock) {
-    s_key[i] = kEmptyWord;
-    s_cnt[i] = 0;
-  }
   __syncthreads();
-  asm volatile("griddepcontrol.wait;" ::: "memory");
 #pragma unroll
   for (int j = 0; j < kRecordKpt; j++) {
     const unsigned same = __match_any_sync(kFull, key[j]);
