@@ -577,6 +577,7 @@ struct Replica {
   std::vector<cudaEvent_t> copy_events;
   uint32_t* stamp = nullptr;               // deduplicated lookups: one stamp per id (first use)
   uint32_t stamp_epoch = 0;
+  uint32_t unique_slot = 0;                // which of Counters::unique_count the next one uses
   int host_order_min_rows = 8192;
   uint64_t lookups_host_ordered = 0;
   uint32_t direct_slot = 0, last_slot = 0; // count slot of the next / the last direct launch
@@ -1060,11 +1061,18 @@ bool choose_direct(const Replica* r) {
   return host <= (uint32_t)r->direct_max_host_rows || remote > host;
 }
 
-// `n_dev` != nullptr: the key count is read on the device from there (at most n); such a lookup
-// always takes the direct extraction and is launched without programmatic overlap, because its
-// keys were produced by the kernels just ahead of it in the stream.
+// What the extraction of a deduplicated lookup needs besides (see DirectParams).
+struct UniqueArgs {
+  const void* batch_keys;
+  int32_t* inverse;
+  uint32_t* n_unique;
+  uint32_t slot;
+};
+
+// `uniq` != nullptr: `keys` are the distinct ones of a batch of n, left by the claim just ahead in the
+// stream together with their number; such a lookup always takes the direct extraction.
 int do_lookup(ugc_ctx* c, Replica* r, const void* keys, int key_bytes, size_t n, void* out,
-              cudaStream_t s, const uint32_t* n_dev = nullptr) {
+              cudaStream_t s, const UniqueArgs* uniq = nullptr) {
   if (n == 0) return UGC_OK;
   if (!keys || !out) return fail(UGC_ERR_INVALID, "keys and out must be non-null");
   if (n > r->max_batch)
@@ -1075,10 +1083,16 @@ int do_lookup(ugc_ctx* c, Replica* r, const void* keys, int key_bytes, size_t n,
   if (prof) UGC_CUDA(cudaEventRecord(r->prof_events[r->prof_used], s));
   // counted before the launch: drain_lookups() must never miss a lookup that could be running
   __atomic_fetch_add(&r->lookups, 1, __ATOMIC_SEQ_CST);
-  if (n_dev != nullptr || choose_direct(r)) {
+  if (uniq != nullptr || choose_direct(r)) {
     if (prof) UGC_CUDA(cudaEventRecord(r->prof_events[r->prof_used + 1], s));
     DirectParams d{};
-    d.n_dev = n_dev;
+    if (uniq) {
+      d.stamp = r->stamp;
+      d.batch_keys = uniq->batch_keys;
+      d.inverse = uniq->inverse;
+      d.n_unique = uniq->n_unique;
+      d.unique_slot = uniq->slot;
+    }
     for (int i = 0; i < kMaxLocation; i++) d.src_base[i] = r->src_base[i];
     d.out = out;
     d.table = r->table;
@@ -1106,7 +1120,7 @@ int do_lookup(ugc_ctx* c, Replica* r, const void* keys, int key_bytes, size_t n,
       early = f->seq != 0 && f->count[kGroupHost] >= 1024u;
     }
     UGC_CUDA(launch_extract_direct(keys, key_bytes, d, r->direct_grid, r->direct_block, r->direct_deep != 0,
-                                   early && d.host_base != nullptr, (r->pdl & 1) != 0 && n_dev == nullptr, s));
+                                   early && d.host_base != nullptr, (r->pdl & 1) != 0, s));
     if (prof) {
       UGC_CUDA(cudaEventRecord(r->prof_events[r->prof_used + 2], s));
       r->prof_used += 3;
@@ -1825,10 +1839,12 @@ int ugc_lookup_unique(ugc_ctx* c, int replica_id, const void* keys, int key_byte
     UGC_CUDA(cudaMemsetAsync(r->stamp, 0, stamp_bytes, s));
     r->stamp_epoch = 1;
   }
-  UGC_CUDA(launch_unique(keys, key_bytes, (uint32_t)n, c->cfg.num_total_item, r->stamp_epoch, r->stamp,
-                         unique_keys, inverse, n_unique, r->counters, s));
-  r->kernel_launches += 2;
-  return do_lookup(c, r, unique_keys, key_bytes, n, out_rows, s, n_unique);
+  const UniqueArgs uniq{keys, inverse, n_unique, r->unique_slot};
+  UGC_CUDA(launch_unique_claim(keys, key_bytes, (uint32_t)n, c->cfg.num_total_item, r->stamp_epoch, r->stamp,
+                               unique_keys, &r->counters->unique_count[uniq.slot], r->counters, (r->pdl & 1) != 0, s));
+  r->unique_slot ^= 1u;
+  r->kernel_launches += 1;
+  return do_lookup(c, r, unique_keys, key_bytes, n, out_rows, s, &uniq);
 }
 
 int ugc_lookup_pool(ugc_ctx* c, int replica_id, const void* keys, int key_bytes, size_t n_keys,

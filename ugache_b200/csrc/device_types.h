@@ -74,7 +74,8 @@ struct Counters {
   // direct extraction: per-source counts of the launches that own slot 0 / slot 1 in turn; a
   // launch adds to its slot and clears the other one (whose launch is complete by then)
   uint32_t dcount[2][kNumGroup];
-  uint32_t reserved3[2];
+  // deduplicated lookups: distinct keys found, in slots used in turn like dcount's
+  uint32_t unique_count[2];
   alignas(16) uint32_t shown[kNumGroup + 1];  // what the pinned mirror shows: counts and ordinal
   // pooled lookups: rows summed so far, per source group (cumulative)
   unsigned long long pool_rows[kNumGroup];
@@ -139,7 +140,13 @@ struct DirectParams {
   TableView table;
   Counters* counters;
   Feedback* feedback;   // pinned host mirror of the last lookup's counts, or nullptr
-  const uint32_t* n_dev;  // if set: the number of keys, in device memory (never above n_keys)
+  // Deduplicated lookup (stamp != nullptr): the keys are the distinct ones of the batch_keys, their
+  // number stands in Counters::unique_count[unique_slot] (n_keys = size of the batch)
+  const uint32_t* stamp;
+  const void* batch_keys;
+  int32_t* inverse;     // out: index of every key of the batch, -1 for an id outside the table
+  uint32_t* n_unique;   // out: number of distinct keys
+  uint32_t unique_slot;
   const void* host_base;  // src_base[host_loc], for the kernel's prologue
   uint32_t n_keys;
   uint32_t row_bytes;
@@ -147,7 +154,7 @@ struct DirectParams {
   uint32_t host_loc;
   uint32_t host_mask;
   uint32_t lpr_shift;   // log2 of the lanes that share one row
-  uint32_t tile_shift;  // log2 of the keys one warp probes at a time (3..5)
+  uint32_t tile_shift;  // log2 of the keys one warp probes at a time; above 5: the kernel chooses
   uint32_t slot;        // which of Counters::dcount this launch adds to (launches alternate)
   uint32_t publish_prev;  // 1: the launch before this one was a direct one; hand its counts on
   uint32_t prev_seq;      // its ordinal among the replica's lookups

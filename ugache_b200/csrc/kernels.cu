@@ -4,7 +4,6 @@
 #include "kernels.cuh"
 
 #include <cuda_fp16.h>
-
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
@@ -696,58 +695,105 @@ __global__ void __launch_bounds__(1024) gather_roles_kernel(GatherParams p) {
 // ------------------------------------------------------------------------------------
 // One 32-bit stamp per id of the key space: {epoch : 8 | index : 24}.  A key is new in this
 // batch when its stamp carries another epoch; the thread that swings the stamp to the current
-// epoch takes the next index and records the key.  A second pass reads the index of every key
-// (the owner may not have stored it yet when another thread of the first pass looks).  No sort,
-// no hashing: the key space is dense and its table already costs 4 bytes per id.
+// epoch takes the next index and records the key.  The index of every key of the batch is read by
+// the extraction that follows (the owner may not have stored it yet when another thread of the claim
+// looks).  No sort: the key space is dense and its table already costs 4 bytes per id.
 constexpr uint32_t kStampPending = 0x00ffffffu;
+
+// What bounded the claim was the L2's rate of operations on ONE address (0.6 ns each): before the
+// first of them lands, every occurrence of the hottest id (18 % of a Zipf-1.2 batch) sees the old
+// stamp and tries to swing it, and each warp took its indices with an addition of its own.  So a
+// CTA's 1024 keys first meet in a direct-mapped set of ids in shared memory, where one occurrence
+// of an id goes on to the L2 (an id whose place is taken goes there itself), and a CTA takes its
+// indices with one addition.  212,992 keys, 29,504 of them distinct, claim,
+// extraction and index together: 45 -> 20.6 us.
+constexpr int kClaimKpt = 4;
+constexpr uint32_t kClaimSlots = 2048;
 
 template <typename KeyT>
 __global__ void __launch_bounds__(kBlock)
     unique_claim_kernel(const KeyT* __restrict__ keys, uint32_t n, uint64_t num_keys, uint32_t epoch,
-                        uint32_t* stamp, KeyT* __restrict__ unique_keys, uint32_t* n_unique,
+                        uint32_t* stamp, KeyT* __restrict__ unique_keys, uint32_t* count,
                         Counters* counters) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t lane = threadIdx.x & 31;
-  bool winner = false;
-  uint64_t k = 0;
-  if (i < n) {
-    k = (uint64_t)keys[i];
-    if (k >= num_keys) {
-      atomicAdd(&counters->err_key_range, 1ull);
-    } else {
-      const uint32_t mine = (epoch << 24) | kStampPending;
-      uint32_t cur = *reinterpret_cast<volatile uint32_t*>(stamp + k);
-      while ((cur >> 24) != epoch) {
-        const uint32_t old = atomicCAS(stamp + k, cur, mine);
-        if (old == cur) {
-          winner = true;
-          break;
-        }
-        cur = old;
-      }
+  __shared__ uint32_t s_key[kClaimSlots];
+  __shared__ uint32_t s_warp[kWarpsPerBlock];
+  __shared__ uint32_t s_base;
+  for (uint32_t i = threadIdx.x; i < kClaimSlots; i += kBlock) s_key[i] = kEmptyWord;
+  // everything is read and written behind the dependency wait: the stamps and the count are the
+  // previous call's, and the keys may be what the launch ahead writes
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t base = blockIdx.x * (kBlock * kClaimKpt) + threadIdx.x;
+  const uint32_t mine = (epoch << 24) | kStampPending;
+  uint32_t key[kClaimKpt], cur[kClaimKpt], bad = 0;
+#pragma unroll
+  for (int j = 0; j < kClaimKpt; j++) {
+    const uint32_t i = base + j * kBlock;
+    const uint64_t k = i < n ? (uint64_t)keys[i] : num_keys;
+    key[j] = k < num_keys ? (uint32_t)k : kEmptyWord;  // also drops negative int64 ids
+    bad += i < n && k >= num_keys;
+  }
+  __syncthreads();  // s_key is clear
+#pragma unroll
+  for (int j = 0; j < kClaimKpt; j++) {
+    cur[j] = mine;
+    if (key[j] != kEmptyWord) cur[j] = *reinterpret_cast<volatile uint32_t*>(stamp + key[j]);
+  }
+  // one occurrence of an id in this CTA goes on
+  bool go[kClaimKpt];
+#pragma unroll
+  for (int j = 0; j < kClaimKpt; j++) {
+    go[j] = (cur[j] >> 24) != epoch;
+    if (go[j]) {
+      volatile uint32_t* slot = s_key + ((key[j] * 2654435761u) >> 21);
+      uint32_t held = *slot;
+      if (held == kEmptyWord) held = atomicCAS(const_cast<uint32_t*>(slot), kEmptyWord, key[j]);
+      go[j] = held != key[j];  // kEmptyWord: this thread's; another id: goes on by itself
     }
   }
-  // one atomic per warp for the indices of its winners
-  const unsigned m = __ballot_sync(kFull, winner);
-  uint32_t base = 0;
-  if (m != 0 && lane == (uint32_t)(__ffs(m) - 1)) base = atomicAdd(n_unique, (uint32_t)__popc(m));
-  base = __shfl_sync(kFull, base, m ? __ffs(m) - 1 : 0);
-  if (winner) {
-    const uint32_t idx = base + __popc(m & ((1u << lane) - 1));
-    unique_keys[idx] = (KeyT)k;
-    atomicExch(stamp + k, (epoch << 24) | idx);
+  uint32_t old[kClaimKpt];
+#pragma unroll
+  for (int j = 0; j < kClaimKpt; j++)
+    if (go[j]) old[j] = atomicCAS(stamp + key[j], cur[j], mine);
+  uint32_t before[kClaimKpt], total = 0;  // winners of this warp ahead of this thread's, per key
+#pragma unroll
+  for (int j = 0; j < kClaimKpt; j++) {
+    if (go[j]) {
+      while (old[j] != cur[j] && (old[j] >> 24) != epoch) {
+        cur[j] = old[j];
+        old[j] = atomicCAS(stamp + key[j], cur[j], mine);
+      }
+      go[j] = old[j] == cur[j];
+    }
+    const unsigned m = __ballot_sync(kFull, go[j]);
+    before[j] = total + __popc(m & ((1u << lane) - 1));
+    total += __popc(m);
+  }
+  if (lane == 0) s_warp[warp] = total;
+  bad = __reduce_add_sync(kFull, bad);
+  if (lane == 0 && bad) atomicAdd(&counters->err_key_range, (unsigned long long)bad);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t run = 0;
+#pragma unroll
+    for (int w = 0; w < kWarpsPerBlock; w++) {
+      const uint32_t c = s_warp[w];
+      s_warp[w] = run;
+      run += c;
+    }
+    s_base = run ? atomicAdd(count, run) : 0;
+  }
+  __syncthreads();
+  const uint32_t first = s_base + s_warp[warp];
+#pragma unroll
+  for (int j = 0; j < kClaimKpt; j++) {
+    if (!go[j]) continue;
+    unique_keys[first + before[j]] = (KeyT)key[j];
+    stamp[key[j]] = (epoch << 24) | (first + before[j]);
   }
 }
-
-template <typename KeyT>
-__global__ void __launch_bounds__(kBlock)
-    unique_inverse_kernel(const KeyT* __restrict__ keys, uint32_t n, uint64_t num_keys,
-                          const uint32_t* __restrict__ stamp, int32_t* __restrict__ inverse) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint64_t k = (uint64_t)keys[i];
-  inverse[i] = k < num_keys ? (int32_t)(stamp[k] & kStampPending) : -1;
-}
+static_assert(kClaimSlots == 1u << 11, "the slot is the top 11 bits of the hash");
 
 // ------------------------------------------------------------------------------------
 // host list in address order
@@ -884,7 +930,29 @@ __device__ __forceinline__ void fetch_key(const KeyT* __restrict__ keys, uint32_
   key = (uint32_t)k;
 }
 
-template <typename KeyT, int VEC, bool FLAT, bool DEEP, bool EARLY>
+// Keys per tile (log2): 32 at first.  A batch that leaves warps without a tile is bound by the chain
+// key - probe - rows of one warp: halve the tile while all tiles still run at once, down to the rows
+// one pass copies (208 keys of 512-byte rows back to back: one pass of 4 rows a warp instead of
+// eight, 6.6 -> 4.3 us).  Then halve it to 8 at least while the warps' tile counts differ by a tenth.
+__host__ __device__ inline uint32_t direct_tile_shift(uint32_t n_keys, uint32_t n_warps, uint32_t rows_per_pass) {
+  uint32_t shift = 5;
+  auto tiles = [&](uint32_t sh) { return (uint32_t)(((uint64_t)n_keys + (1u << sh) - 1) >> sh); };
+  while (shift > 0 && (1u << (shift - 1)) >= rows_per_pass && tiles(shift - 1) <= n_warps) shift--;
+  while (shift > 3 && (1u << (shift - 1)) >= rows_per_pass) {
+    const uint32_t t = tiles(shift);
+    const uint32_t rounds = (t + n_warps - 1) / n_warps;
+    if (t <= n_warps || 10ull * t >= 9ull * rounds * n_warps) break;
+    shift--;
+  }
+  return shift;
+}
+
+// UNIQUE: the extraction of a deduplicated lookup.  Its keys, their number and the stamps come from
+// the claim just ahead in the stream, so it waits first; the tile size follows the number found; and
+// it writes the index of every key of the batch, whose loads go out with the first probes instead of
+// in a launch of their own.  It lets nothing start early: what it writes besides rows (the index, the
+// number) may be the next launch's keys.
+template <typename KeyT, int VEC, bool FLAT, bool DEEP, bool EARLY, bool UNIQUE>
 __global__ void __launch_bounds__(kBlock, DEEP ? 3 : 4)
     extract_direct_kernel(const KeyT* __restrict__ keys, DirectParams p) {
   // rows in flight per lane group: 4 (2 with 32-byte vectors) at 4 CTAs per SM, or twice that
@@ -898,10 +966,21 @@ __global__ void __launch_bounds__(kBlock, DEEP ? 3 : 4)
   }
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t n_warps = gridDim.x * (blockDim.x >> 5);
-  const uint32_t tshift = p.tile_shift;
+  uint32_t n_keys = p.n_keys, tshift = p.tile_shift;
+  uint32_t inv_at = 0, inv_step = 0;
+  uint64_t inv_key[2] = {0, 0};
+  if (UNIQUE) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    n_keys = min(__ldcg(&p.counters->unique_count[p.unique_slot]), p.n_keys);
+    if (tshift > 5) tshift = direct_tile_shift(n_keys, n_warps, min(32u, UNROLL * (32u >> p.lpr_shift)));
+    inv_at = blockIdx.x * blockDim.x + threadIdx.x;
+    inv_step = gridDim.x * blockDim.x;
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+      if (inv_at + j * inv_step < p.n_keys)
+        inv_key[j] = (uint64_t)static_cast<const KeyT*>(p.batch_keys)[inv_at + j * inv_step];
+  }
   const uint32_t tile_keys = 1u << tshift;
-  // the number of keys may live in device memory (distinct keys of a batch, counted on the GPU)
-  const uint32_t n_keys = p.n_dev ? min(*p.n_dev, p.n_keys) : p.n_keys;
   const uint32_t n_tiles = (n_keys + tile_keys - 1) >> tshift;
   uint32_t tile = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   if (threadIdx.x < kNumGroup) s_cnt[threadIdx.x] = 0;
@@ -916,7 +995,15 @@ __global__ void __launch_bounds__(kBlock, DEEP ? 3 : 4)
   fetch_key(keys, tile + n_warps, n_tiles, tshift, n_keys, p.table.num_keys, lane, key_nxt, ok_nxt, bad);
   Probe<FLAT> pr;
   probe_issue(p.table, key_cur, ok_cur, pr);
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (!UNIQUE) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  auto batch_index = [&](uint64_t k) {  // index of an id of the batch among the distinct ones
+    return k < p.table.num_keys ? (int32_t)(__ldcg(p.stamp + k) & kStampPending) : -1;
+  };
+  int32_t inv_idx[2];
+  if (UNIQUE) {
+#pragma unroll
+    for (int j = 0; j < 2; j++) inv_idx[j] = batch_index(inv_key[j]);
+  }
   uint32_t word = probe_resolve(p.table, pr, key_cur, ok_cur);
   // EARLY: the first host row of this warp's first tile is fetched before the dependency wait
   // (the host table is never written by a lookup) and held in registers, one piece per lane.
@@ -969,8 +1056,18 @@ __global__ void __launch_bounds__(kBlock, DEEP ? 3 : 4)
       p.counters->t_start = t0;
       p.counters->t_index = 0;
       p.counters->last_keys = p.n_keys;
+      if (UNIQUE) {
+        *p.n_unique = n_keys;
+        p.counters->unique_count[p.unique_slot ^ 1u] = 0;  // for the next deduplicated lookup
+      }
     }
   };
+  if (UNIQUE) {
+    wait_for_launch_ahead();
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+      if (inv_at + j * inv_step < p.n_keys) p.inverse[inv_at + j * inv_step] = inv_idx[j];
+  }
 
   const uint32_t lpr = 1u << p.lpr_shift;
   const uint32_t rpi = 32u >> p.lpr_shift;       // rows per warp-wide load
@@ -1043,6 +1140,9 @@ __global__ void __launch_bounds__(kBlock, DEEP ? 3 : 4)
   }
 
   if (!waited) wait_for_launch_ahead();  // a warp without rows
+  if (UNIQUE)
+    for (uint32_t i = inv_at + 2 * inv_step; i < p.n_keys; i += inv_step)
+      p.inverse[i] = batch_index((uint64_t)static_cast<const KeyT*>(p.batch_keys)[i]);
   // Per-source counts of this lookup: fire-and-forget adds into the slot this launch owns.
   // Nothing here waits on memory, so the kernel ends with its last row store: no count of
   // finished CTAs, no fence, no single CTA that tidies up after the others.
@@ -1766,29 +1866,14 @@ cudaError_t launch_extract_direct(const void* keys, int key_bytes, const DirectP
   const int lpr = lanes_per_row(p.row_bytes, vec);
   p.lpr_shift = 0;
   while ((1 << p.lpr_shift) < lpr) p.lpr_shift++;
-  // Tile size: the largest of 32 / 16 / 8 keys (never less than the rows one pass of a warp
-  // copies) with which the warps' tile counts differ by less than a tenth; forced by
-  // p.tile_shift when that is set.
-  const int unroll = (vec == 32 ? 2 : 4) * (deep ? 2 : 1);
-  const int rows_per_pass = std::min(32, unroll * (32 / lpr));
-  const long long n_warps = (long long)grid * warps_per_block;
+  // p.tile_shift 3..5 forces the tile
+  const int unroll = (vec == 32 ? 2 : 4) * (deep && !p.stamp ? 2 : 1);
   uint32_t shift = p_in.tile_shift;
-  if (shift < 3 || shift > 5) {
-    shift = 5;
-    // A batch that leaves warps without a tile is bound by the chain key - probe - rows of one warp:
-    // halve the tile while all tiles still run at once, down to the rows one pass copies (208 keys
-    // of 512-byte rows back to back: one pass of 4 rows a warp instead of eight, 6.6 -> 4.3 us).
-    while (shift > 0 && (1 << (shift - 1)) >= rows_per_pass &&
-           (((long long)p.n_keys + (1ll << (shift - 1)) - 1) >> (shift - 1)) <= n_warps)
-      shift--;
-    while (shift > 3 && (1 << (shift - 1)) >= rows_per_pass) {
-      const long long tiles = ((long long)p.n_keys + (1ll << shift) - 1) >> shift;
-      const long long rounds = (tiles + n_warps - 1) / n_warps;
-      if (tiles <= n_warps || (double)tiles / (double)(rounds * n_warps) >= 0.9) break;
-      shift--;
-    }
-  }
   p.tile_shift = shift;
+  if (shift < 3 || shift > 5) {
+    shift = direct_tile_shift(p.n_keys, (uint32_t)(grid * warps_per_block), (uint32_t)std::min(32, unroll * (32 / lpr)));
+    p.tile_shift = p.stamp ? 32u : shift;  // of a deduplicated lookup the kernel knows the number of keys
+  }
   const int tiles = (int)(((long long)p.n_keys + (1ll << shift) - 1) >> shift);
   grid = std::max(1, std::min(grid, (tiles + warps_per_block - 1) / warps_per_block));
   auto launch = [&](auto key, auto vec_c, auto flat_c) {
@@ -1796,10 +1881,12 @@ cudaError_t launch_extract_direct(const void* keys, int key_bytes, const DirectP
     constexpr int V = decltype(vec_c)::value;
     constexpr bool F = decltype(flat_c)::value;
     const KeyT* k = static_cast<const KeyT*>(keys);
-    if (deep) return launch_pdl(extract_direct_kernel<KeyT, V, F, true, false>, grid, block, 0, stream, pdl, k, p);
+    if (p.stamp)
+      return launch_pdl(extract_direct_kernel<KeyT, V, F, false, false, true>, grid, block, 0, stream, pdl, k, p);
+    if (deep) return launch_pdl(extract_direct_kernel<KeyT, V, F, true, false, false>, grid, block, 0, stream, pdl, k, p);
     if (early_host)
-      return launch_pdl(extract_direct_kernel<KeyT, V, F, false, true>, grid, block, 0, stream, pdl, k, p);
-    return launch_pdl(extract_direct_kernel<KeyT, V, F, false, false>, grid, block, 0, stream, pdl, k, p);
+      return launch_pdl(extract_direct_kernel<KeyT, V, F, false, true, false>, grid, block, 0, stream, pdl, k, p);
+    return launch_pdl(extract_direct_kernel<KeyT, V, F, false, false, false>, grid, block, 0, stream, pdl, k, p);
   };
   auto by_table = [&](auto key, auto vec_c) {
     return p.table.kind == kTableFlat ? launch(key, vec_c, std::true_type{}) : launch(key, vec_c, std::false_type{});
@@ -1870,26 +1957,16 @@ cudaError_t launch_lookup_pool(const void* keys, int key_bytes, const PoolParams
   return cudaGetLastError();
 }
 
-cudaError_t launch_unique(const void* keys, int key_bytes, uint32_t n, uint64_t num_keys, uint32_t epoch,
-                          uint32_t* stamp, void* unique_keys, int32_t* inverse, uint32_t* n_unique,
-                          Counters* counters, cudaStream_t stream) {
-  if (n == 0) return cudaMemsetAsync(n_unique, 0, sizeof(uint32_t), stream);
-  cudaError_t e = cudaMemsetAsync(n_unique, 0, sizeof(uint32_t), stream);
-  if (e != cudaSuccess) return e;
-  if (key_bytes == 8) {
-    unique_claim_kernel<long long><<<grid_for(n), kBlock, 0, stream>>>(
-        static_cast<const long long*>(keys), n, num_keys, epoch, stamp, static_cast<long long*>(unique_keys),
-        n_unique, counters);
-    unique_inverse_kernel<long long><<<grid_for(n), kBlock, 0, stream>>>(static_cast<const long long*>(keys), n,
-                                                                         num_keys, stamp, inverse);
-  } else {
-    unique_claim_kernel<uint32_t><<<grid_for(n), kBlock, 0, stream>>>(
-        static_cast<const uint32_t*>(keys), n, num_keys, epoch, stamp, static_cast<uint32_t*>(unique_keys),
-        n_unique, counters);
-    unique_inverse_kernel<uint32_t><<<grid_for(n), kBlock, 0, stream>>>(static_cast<const uint32_t*>(keys), n,
-                                                                        num_keys, stamp, inverse);
-  }
-  return cudaGetLastError();
+cudaError_t launch_unique_claim(const void* keys, int key_bytes, uint32_t n, uint64_t num_keys, uint32_t epoch,
+                                uint32_t* stamp, void* unique_keys, uint32_t* count, Counters* counters, bool pdl,
+                                cudaStream_t stream) {
+  if (n == 0) return cudaSuccess;
+  const int grid = (int)(((uint64_t)n + kBlock * kClaimKpt - 1) / (kBlock * kClaimKpt));
+  if (key_bytes == 8)
+    return launch_pdl(unique_claim_kernel<long long>, grid, kBlock, 0, stream, pdl, static_cast<const long long*>(keys),
+                      n, num_keys, epoch, stamp, static_cast<long long*>(unique_keys), count, counters);
+  return launch_pdl(unique_claim_kernel<uint32_t>, grid, kBlock, 0, stream, pdl, static_cast<const uint32_t*>(keys), n,
+                    num_keys, epoch, stamp, static_cast<uint32_t*>(unique_keys), count, counters);
 }
 
 size_t host_order_scratch_bytes() { return 2 * kHostBuckets * sizeof(uint32_t); }

@@ -33,13 +33,14 @@ cudaError_t launch_lookup_group(const void* keys, int key_bytes, uint32_t n, con
 cudaError_t launch_gather_roles(const GatherParams& p, int grid, int block, int vec_bytes,
                                 cudaStream_t stream);
 
-// Distinct keys of a batch: unique_keys[0 .. *n_unique) (order of discovery), inverse[i] = index
-// of keys[i] among them (-1 for an id outside [0, num_keys)).  `stamp` is one uint32 per id of
-// the key space, zeroed once; `epoch` (1..255) must differ from the one of the previous call on
-// the same stamp array and the array be zeroed again before an epoch value comes round.
-cudaError_t launch_unique(const void* keys, int key_bytes, uint32_t n, uint64_t num_keys, uint32_t epoch,
-                          uint32_t* stamp, void* unique_keys, int32_t* inverse, uint32_t* n_unique,
-                          Counters* counters, cudaStream_t stream);
+// Distinct keys of a batch: unique_keys[0 .. *count) in order of discovery; `count` is zero on entry.
+// `stamp` is one uint32 per id of the key space, zeroed once; `epoch` (1..255) must differ from the
+// one of the previous call on the same stamp array and the array be zeroed again before an epoch
+// value comes round.  launch_extract_direct with DirectParams::stamp set follows: it extracts the
+// rows of the distinct keys and writes the index of every key of the batch among them.
+cudaError_t launch_unique_claim(const void* keys, int key_bytes, uint32_t n, uint64_t num_keys, uint32_t epoch,
+                                uint32_t* stamp, void* unique_keys, uint32_t* count, Counters* counters, bool pdl,
+                                cudaStream_t stream);
 
 // Pooled lookup: out[b] = sum (or mean) over the keys of bag b of their rows, fp32, added in key
 // order.  Rows must be a multiple of 16 bytes and every source and `out` 16-byte aligned.
