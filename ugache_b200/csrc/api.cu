@@ -1888,7 +1888,8 @@ int ugc_lookup_pool(ugc_ctx* c, int replica_id, const void* keys, int key_bytes,
   p.host_loc = (uint32_t)c->cfg.num_device;
   p.host_mask = host_mask_value(c->cfg.empty_feat);
   p.mean = mode == UGC_POOL_MEAN ? 1u : 0u;
-  UGC_CUDA(launch_lookup_pool(keys, key_bytes, p, elem_type == UGC_ELEM_F16, r->sm_count * 8, r->pool_vec_bytes, s));
+  UGC_CUDA(launch_lookup_pool(keys, key_bytes, p, elem_type == UGC_ELEM_F16, r->sm_count, r->pool_vec_bytes,
+                              (r->pdl & 1) != 0, s));
   r->kernel_launches += 1;
   r->lookups_pooled++;
   remember_stream(r, s);

@@ -3,7 +3,6 @@
 // is not a multiple of 16).
 #include "kernels.cuh"
 
-#include <cuda_fp16.h>
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
@@ -1163,23 +1162,37 @@ __global__ void __launch_bounds__(kBlock, DEEP ? 3 : 4)
 // pooled lookup: table probe, row fetch and per-bag sum in ONE kernel
 // ------------------------------------------------------------------------------------
 // A bag is a run of consecutive keys; its result is the sum (or mean) of its rows, one fp32
-// vector of `dim` elements.  The looked-up rows never reach memory: a group of lanes (as many
-// as a row has 16-byte pieces, at most 32) owns a bag, each lane probes the table for one key of
-// the bag, the row addresses travel by shuffle inside the group, and every lane adds up its
-// own 16-byte column of the rows.  The additions of one output element happen in key order,
-// in fp32, starting from +0, one rounding each (no fused multiply-add is involved), so the
-// result is bit-for-bit what a sequential fp32 loop over the bag gives on any machine.
-// Keys outside [0, num_keys) are counted and contribute nothing.  The reference leaves pooling
-// to the model that consumes the rows; this is the fused form of lookup + segment sum.
+// vector of `dim` elements.  The looked-up rows never reach memory.  The additions of one output
+// element happen in key order, in fp32, starting from +0, one rounding each (no fused multiply-add
+// is involved), so the result is bit-for-bit what a sequential fp32 loop over the bag gives on any
+// machine.  Keys outside [0, num_keys) are counted and contribute nothing.  The reference leaves
+// pooling to the model that consumes the rows; this is the fused form of lookup + segment sum.
+//
+// What bounds it is latency: offsets - keys - table - rows is a chain of reads, and the order of the
+// additions leaves a bag to the lanes that own its columns.  So
+//  * a CTA is as many warps as a row has columns of 32 pieces; it takes a tile of consecutive bags,
+//    and its threads probe all of the tile's keys at once (two a thread, addresses through shared
+//    memory) instead of each lane group its own bag's;
+//  * 4-byte pieces put four times the warps on a bag and hold 64 rows of it in flight per lane, at four
+//    times the instructions; with 16-byte pieces it is 8 rows;
+//  * the loads run on over the ends of bags, and a bag's end is rare code outside the row loop.
+// Before (a lane group probed and summed bag by bag) and now: 8192 ragged bags of 26 rows of 512 bytes
+// 51 -> 22 us, 65,536 bags of 5 fp16 rows of 128 bytes 23.6 -> 15.7, 73 bags of 400 rows of 1 KiB
+// 167 -> 32, 145 bags of 877 rows of 256 bytes 108 -> 20, 186 bags of 23 rows of 128 bytes 15 -> 6.4.
+// With 16-byte pieces and many bags the rows' way through the L1 and the instructions bound it.
 template <bool F16, int VEC>
 __device__ __forceinline__ void pool_add(float* acc, const Vec<VEC>& v) {
   if (F16) {
-    const __half2* h = reinterpret_cast<const __half2*>(&v);
 #pragma unroll
     for (int i = 0; i < VEC / 4; i++) {
-      const float2 f = __half22float2(h[i]);
-      acc[2 * i] = __fadd_rn(acc[2 * i], f.x);
-      acc[2 * i + 1] = __fadd_rn(acc[2 * i + 1], f.y);
+      // volatile: the widened values of many rows in flight would not fit the registers, and moving
+      // the conversion out of a loop over the bags that share those rows is what the compiler does
+      float x, y;
+      asm volatile("{\n\t.reg .f16 a, b;\n\tmov.b32 {a, b}, %2;\n\tcvt.f32.f16 %0, a;\n\tcvt.f32.f16 %1, b;\n\t}"
+                   : "=f"(x), "=f"(y)
+                   : "r"(v.v[i]));
+      acc[2 * i] = __fadd_rn(acc[2 * i], x);
+      acc[2 * i + 1] = __fadd_rn(acc[2 * i + 1], y);
     }
   } else {
     const float* f = reinterpret_cast<const float*>(&v);
@@ -1194,148 +1207,164 @@ __device__ __forceinline__ uint32_t pool_bag_start(const PoolParams& p, uint32_t
   return (uint32_t)min(max(o, 0ll), (long long)p.n_keys);
 }
 
-template <typename KeyT, bool F16, int VEC>
-__global__ void __launch_bounds__(kBlock, 3) lookup_pool_kernel(const KeyT* __restrict__ keys, PoolParams p) {
-  constexpr int NF = VEC / (F16 ? 2 : 4);  // elements per piece of a row (VEC bytes)
-  constexpr int UNROLL = VEC == 16 ? 8 : 16;  // rows in flight per lane
-  __shared__ const char* s_src[kMaxLocation];
-  if (threadIdx.x < kMaxLocation) s_src[threadIdx.x] = static_cast<const char*>(p.src_base[threadIdx.x]);
-  __syncthreads();
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t lpr = 1u << p.lpr_shift;
-  const uint32_t sub = lane & (lpr - 1);
-  const uint32_t gbase = lane & ~(lpr - 1);
-  const unsigned gmask = lpr == 32 ? kFull : (((1u << lpr) - 1u) << gbase);
-  const uint32_t workers_per_cta = blockDim.x >> p.lpr_shift;
-  const uint32_t n_workers = gridDim.x * workers_per_cta;
-  const uint32_t vecs = p.row_bytes / VEC;
-  const uint32_t n_tiles = (p.n_bags + p.bags_per_tile - 1) / p.bags_per_tile;
-  // rows wider than one lane group (32 pieces) are cut into column passes; a pass over a tile
-  // is the unit of work, so that wide rows (or, with 4-byte pieces, every row) spread a bag
-  // over several lane groups
-  const uint32_t n_pass = (vecs + lpr - 1) >> p.lpr_shift;
-  const uint32_t n_items = n_tiles * n_pass;
-  uint32_t bad = 0, n_local = 0, n_remote = 0, n_host = 0;
+constexpr int kPoolMaxBlock = 256;  // eight columns; wider rows take several CTAs a tile
+constexpr uint32_t kPoolMaxBags = 128;  // bags a tile
 
-  // A lane group owns a tile of consecutive bags (several when bags are shorter than the group
-  // is wide, so that every lane has a key to probe) and walks the tile's keys in order: probe
-  // `lpr` keys, fetch their rows UNROLL at a time, add them up in key order, and write a bag out
-  // whenever the walk crosses into the next one.
-  for (uint32_t item = blockIdx.x * workers_per_cta + (threadIdx.x >> p.lpr_shift); item < n_items;
-       item += n_workers) {
-    const uint32_t tile = item / n_pass;
-    const uint32_t c0 = (item - tile * n_pass) << p.lpr_shift;
-    const uint32_t bag_lo = tile * p.bags_per_tile;
-    const uint32_t bag_hi = min(bag_lo + p.bags_per_tile, p.n_bags);
-    const uint32_t k_lo = pool_bag_start(p, bag_lo);
-    const uint32_t k_hi = max(k_lo, pool_bag_start(p, bag_hi));
-    {
-      const uint32_t c = c0 + sub;
-      const bool has = c < vecs;
-      float acc[NF];
+template <typename KeyT, bool F16, int VEC>
+__global__ void __launch_bounds__(kPoolMaxBlock, VEC == 16 ? 3 : 2) lookup_pool_kernel(const KeyT* __restrict__ keys, PoolParams p) {
+  constexpr int NF = VEC / (F16 ? 2 : 4);  // elements per piece of a row (VEC bytes)
+  constexpr uint32_t UNROLL = VEC == 16 ? 8 : 64;  // rows in flight per lane
+  constexpr int KPT = 2;                   // keys a thread probes at a time
+  __shared__ const char* s_src[kMaxLocation];
+  __shared__ const char* s_row[KPT * kPoolMaxBlock];  // rows of the chunk of keys at hand; nullptr: none
+  __shared__ uint32_t s_end[kPoolMaxBags + 1];        // where the tile's bags start, and the last one ends
+  __shared__ uint32_t s_cnt[kNumGroup + 1];
+  const uint32_t tid = threadIdx.x;
+  if (tid < kMaxLocation) s_src[tid] = static_cast<const char*>(p.src_base[tid]);
+  if (tid <= kNumGroup) s_cnt[tid] = 0;
+  // nothing is read ahead of the dependency wait: keys and offsets may be what the launch ahead writes
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+  const uint32_t tile = blockIdx.x / p.col_blocks, col_block = blockIdx.x - tile * p.col_blocks;
+  const uint32_t bag_lo = tile * p.bags_per_tile;
+  const uint32_t n_bags = min(p.bags_per_tile, p.n_bags - bag_lo);
+  for (uint32_t i = tid; i <= n_bags; i += blockDim.x) s_end[i] = pool_bag_start(p, bag_lo + i);
+  __syncthreads();
+  const uint32_t k_lo = s_end[0];
+  const uint32_t k_hi = max(k_lo, s_end[n_bags]);
+
+  // a lane group (as many lanes as a column has pieces) adds up one column of the bags
+  // [bag, bag_hi) of the tile; rows of less than 32 pieces leave a warp several groups, which
+  // share out the tile's bags
+  const uint32_t lpr = 1u << p.lpr_shift;
+  const uint32_t groups = 32u >> p.lpr_shift;
+  const uint32_t group = (tid & 31) >> p.lpr_shift;
+  const uint32_t c = ((col_block * (blockDim.x >> 5) + (tid >> 5)) << p.lpr_shift) + (tid & (lpr - 1));
+  const bool has = c < p.row_bytes / VEC;
+  uint32_t bag = n_bags * group / groups;
+  const uint32_t bag_hi = n_bags * (group + 1) / groups;
+  uint32_t bag_begin = min(max(s_end[bag], k_lo), k_hi);
+  uint32_t bag_end = bag < bag_hi ? max(bag_begin, min(s_end[bag + 1], k_hi)) : bag_begin;
+  uint32_t k = bag_begin;                                               // the group's next key
+  const uint32_t k_end = max(k, min(s_end[bag_hi], k_hi));              // and the end of its keys
+  float acc[NF];
 #pragma unroll
-      for (int i = 0; i < NF; i++) acc[i] = 0.f;
-      uint32_t bag = bag_lo;
-      uint32_t bag_begin = k_lo;
-      uint32_t bag_end = max(bag_begin, min(pool_bag_start(p, bag + 1), k_hi));
-      // writes bag `bag` out and moves on to the next one of the tile
-      auto flush = [&]() {
-        if (has) {
-          const uint32_t len = bag_end - bag_begin;
-          if (p.mean && len > 0) {
-            const float d = (float)len;
+  for (int i = 0; i < NF; i++) acc[i] = 0.f;
+  // writes bag `bag` out and moves on to the next one
+  auto flush = [&]() {
+    if (has) {
+      const uint32_t len = bag_end - bag_begin;
+      if (p.mean && len > 0) {
+        const float d = (float)len;
 #pragma unroll
-            for (int i = 0; i < NF; i++) acc[i] = __fdiv_rn(acc[i], d);
-          }
-          float* dst = p.out + (size_t)bag * p.dim + (size_t)c * NF;
-          if (NF >= 4) {
+        for (int i = 0; i < NF; i++) acc[i] = __fdiv_rn(acc[i], d);
+      }
+      float* dst = p.out + (size_t)(bag_lo + bag) * p.dim + (size_t)c * NF;
+      if (NF >= 4) {
 #pragma unroll
-            for (int i = 0; i + 3 < NF; i += 4)
-              reinterpret_cast<float4*>(dst)[i / 4] = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
-          } else if (NF == 2) {
-            *reinterpret_cast<float2*>(dst) = make_float2(acc[0], acc[NF - 1]);
+        for (int i = 0; i + 3 < NF; i += 4)
+          reinterpret_cast<float4*>(dst)[i / 4] = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+      } else if (NF == 2) {
+        *reinterpret_cast<float2*>(dst) = make_float2(acc[0], acc[NF - 1]);
+      } else {
+        dst[0] = acc[0];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NF; i++) acc[i] = 0.f;
+    bag++;
+    bag_begin = bag_end;
+    if (bag < bag_hi) bag_end = max(bag_begin, min(s_end[bag + 1], k_hi));
+  };
+
+  uint32_t bad = 0, n_local = 0, n_remote = 0, n_host = 0;
+  const uint32_t chunk = KPT * blockDim.x;
+  for (uint32_t c0 = k_lo; c0 < k_hi; c0 += chunk) {
+    uint64_t key[KPT];
+#pragma unroll
+    for (int j = 0; j < KPT; j++) {
+      const uint32_t i = c0 + j * blockDim.x + tid;
+      key[j] = i < k_hi ? (uint64_t)keys[i] : 0;
+    }
+    uint32_t word[KPT];
+#pragma unroll
+    for (int j = 0; j < KPT; j++) {
+      word[j] = kEmptyWord;
+      if (c0 + j * blockDim.x + tid < k_hi && key[j] < p.table.num_keys) word[j] = table_lookup(p.table, (uint32_t)key[j]);
+    }
+    if (c0 != k_lo) __syncthreads();  // every group is done with the chunk before
+#pragma unroll
+    for (int j = 0; j < KPT; j++) {
+      const char* src = nullptr;
+      if (c0 + j * blockDim.x + tid < k_hi) {
+        if (key[j] >= p.table.num_keys) {  // also catches negative int64 ids
+          bad++;
+        } else if (word[j] == kEmptyWord) {
+          src = s_src[p.host_loc] + (size_t)((uint32_t)key[j] & p.host_mask) * p.row_bytes;
+          n_host++;
+        } else {
+          const uint32_t loc = word_loc(word[j]);
+          src = s_src[loc] + (size_t)word_off(word[j]) * p.row_bytes;
+          if (loc == p.local_loc) {
+            n_local++;
           } else {
-            dst[0] = acc[0];
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < NF; i++) acc[i] = 0.f;
-        bag++;
-        bag_begin = bag_end;
-        if (bag < bag_hi) bag_end = max(bag_begin, min(pool_bag_start(p, bag + 1), k_hi));
-      };
-      for (uint32_t k0 = k_lo; k0 < k_hi; k0 += lpr) {
-        // this lane's key: source address of its row
-        const uint32_t idx = k0 + sub;
-        bool valid = idx < k_hi;
-        unsigned long long k = valid ? (unsigned long long)keys[idx] : 0ull;
-        if (k >= p.table.num_keys) {  // also catches negative int64 ids
-          if (valid && c0 == 0) bad++;
-          valid = false;
-        }
-        const char* src = nullptr;
-        if (valid) {
-          const uint32_t w = table_lookup(p.table, (uint32_t)k);
-          uint32_t loc, off;
-          if (w == kEmptyWord) {
-            loc = p.host_loc;
-            off = (uint32_t)k & p.host_mask;
-            if (c0 == 0) n_host++;
-          } else {
-            loc = word_loc(w);
-            off = word_off(w);
-            if (c0 == 0) {
-              if (loc == p.local_loc) {
-                n_local++;
-              } else {
-                n_remote++;
-              }
-            }
-          }
-          src = s_src[loc] + (size_t)off * p.row_bytes;
-        }
-        const unsigned long long src_bits = reinterpret_cast<unsigned long long>(src);
-        const uint32_t cnt = min(lpr, k_hi - k0);
-        for (uint32_t j = 0; j < cnt; j += UNROLL) {
-          Vec<VEC> v[UNROLL];
-          bool ok[UNROLL];
-#pragma unroll
-          for (int u = 0; u < UNROLL; u++) {
-            const unsigned long long a = __shfl_sync(gmask, src_bits, gbase + ((j + u) & (lpr - 1)));
-            ok[u] = has && j + u < cnt && a != 0ull;
-            if (ok[u]) ld_row(v[u], reinterpret_cast<const char*>(a) + (size_t)c * VEC);
-          }
-#pragma unroll
-          for (int u = 0; u < UNROLL; u++) {
-            if (j + u < cnt) {
-              while (k0 + j + u >= bag_end && bag < bag_hi) flush();  // also passes empty bags
-              if (ok[u]) pool_add<F16, VEC>(acc, v[u]);
-            }
+            n_remote++;
           }
         }
       }
-      while (bag < bag_hi) flush();  // the last bag of the tile, and empty ones after it
+      s_row[j * blockDim.x + tid] = src;
+    }
+    __syncthreads();
+    const uint32_t stop = min(k_end, c0 + chunk);
+    for (; k < stop; k += min(UNROLL, stop - k)) {
+      Vec<VEC> v[UNROLL];
+#pragma unroll
+      for (uint32_t u = 0; u < UNROLL; u++) {
+        // a row that is not there adds +0, which leaves a sum that started from +0 as it is
+#pragma unroll
+        for (int i = 0; i < VEC / 4; i++) v[u].v[i] = 0;
+        const char* src = k + u < stop ? s_row[k + u - c0] : nullptr;
+        if (has && src) ld_row(v[u], src + (size_t)c * VEC);
+      }
+      // the part of these rows that lies in the bag at hand, then the bag's end, and on: the end of
+      // a bag stands here once, not behind every row (it is long, and instructions are what small
+      // pieces spend their time on)
+      const uint32_t n = min(UNROLL, stop - k);
+      if (bag_end - k >= n) {
+#pragma unroll
+        for (uint32_t u = 0; u < UNROLL; u++) pool_add<F16, VEC>(acc, v[u]);
+      } else {
+        for (uint32_t lo = 0;;) {
+          const uint32_t hi = min(n, bag_end - k);
+#pragma unroll
+          for (uint32_t u = 0; u < UNROLL; u++)
+            if (u >= lo && u < hi) pool_add<F16, VEC>(acc, v[u]);
+          lo = hi;
+          if (hi >= n || bag >= bag_hi) break;
+          flush();  // also passes empty bags
+        }
+      }
     }
   }
+  while (bag < bag_hi) flush();  // the last bag, and empty ones after it
+
   // counts: one global atomic per CTA and counter (an atomic per thread on one address would
   // take longer than the kernel's memory traffic)
-  __shared__ uint32_t s_cnt[kNumGroup + 1];
-  if (threadIdx.x <= kNumGroup) s_cnt[threadIdx.x] = 0;
-  __syncthreads();
+  if (col_block != 0) return;
   n_local = __reduce_add_sync(kFull, n_local);
   n_remote = __reduce_add_sync(kFull, n_remote);
   n_host = __reduce_add_sync(kFull, n_host);
   bad = __reduce_add_sync(kFull, bad);
-  if (lane == 0) {
+  if ((tid & 31) == 0) {
     if (n_local) atomicAdd(&s_cnt[kGroupLocal], n_local);
     if (n_remote) atomicAdd(&s_cnt[kGroupRemote], n_remote);
     if (n_host) atomicAdd(&s_cnt[kGroupHost], n_host);
     if (bad) atomicAdd(&s_cnt[kNumGroup], bad);
   }
   __syncthreads();
-  if (threadIdx.x < kNumGroup && s_cnt[threadIdx.x])
-    atomicAdd(&p.counters->pool_rows[threadIdx.x], (unsigned long long)s_cnt[threadIdx.x]);
-  if (threadIdx.x == kNumGroup && s_cnt[kNumGroup])
+  if (tid < kNumGroup && s_cnt[tid]) atomicAdd(&p.counters->pool_rows[tid], (unsigned long long)s_cnt[tid]);
+  if (tid == kNumGroup && s_cnt[kNumGroup])
     atomicAdd(&p.counters->err_key_range, (unsigned long long)s_cnt[kNumGroup]);
 }
 
@@ -1899,62 +1928,40 @@ cudaError_t launch_extract_direct(const void* keys, int key_bytes, const DirectP
   return key_bytes == 8 ? by_vec((long long)0) : by_vec((uint32_t)0);
 }
 
-namespace {
-// Launch shape of the pooled lookup for pieces of `vec` bytes: lanes per group, bags per tile,
-// and the number of warps the batch fills.
-struct PoolShape {
-  uint32_t lpr_shift, bags_per_tile, warps;
-};
-PoolShape pool_shape(const PoolParams& p, int vec) {
-  PoolShape sh{};
-  const int lpr = lanes_per_row(p.row_bytes, vec);
-  while ((1 << sh.lpr_shift) < lpr) sh.lpr_shift++;
-  // bags per lane group: as many as it takes to give every lane of the group a key to probe
-  const uint64_t avg_bag = std::max<uint64_t>(1, p.offsets ? (uint64_t)p.n_keys / p.n_bags : p.bag_size);
-  sh.bags_per_tile = (uint32_t)std::max<uint64_t>(1, (uint64_t)lpr / avg_bag);
-  const uint64_t n_tiles = ((uint64_t)p.n_bags + sh.bags_per_tile - 1) / sh.bags_per_tile;
-  const uint64_t n_pass = (p.row_bytes / (uint32_t)vec + lpr - 1) / lpr;
-  sh.warps = (uint32_t)std::min<uint64_t>((n_tiles * n_pass * lpr + 31) / 32, 0xffffffffu);
-  return sh;
-}
-}  // namespace
-
 cudaError_t launch_lookup_pool(const void* keys, int key_bytes, const PoolParams& p_in, bool f16,
-                               int max_ctas, int vec_bytes, cudaStream_t stream) {
+                               int sm_count, int vec_bytes, bool pdl, cudaStream_t stream) {
   if (p_in.n_bags == 0) return cudaSuccess;
   PoolParams p = p_in;
-  // 16-byte pieces unless the batch then fills fewer than two warps per SM (few, very long
-  // bags): 4-byte pieces put four times as many lane groups on a bag and keep twice as many
-  // rows in flight per lane, at four times the probes and load instructions (measured on
-  // 212,992 keys of 512-byte rows: bags of 1024 keys 152 against 200 us, bags of 128 keys 51
-  // against 33 us)
-  PoolShape sh = pool_shape(p, 16);
-  int vec = 16;
-  if (vec_bytes == 4 || (vec_bytes != 16 && sh.warps < (uint32_t)max_ctas * (kBlock / 32) / 32)) {
-    vec = 4;
-    sh = pool_shape(p, 4);
-  }
-  p.lpr_shift = sh.lpr_shift;
-  p.bags_per_tile = sh.bags_per_tile;
-  const int grid = (int)std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)max_ctas,
-                                                                 (sh.warps + kBlock / 32 - 1) / (kBlock / 32)));
-#define UGC_LAUNCH_POOL(KEYT, F16, VEC) \
-  lookup_pool_kernel<KEYT, F16, VEC><<<grid, kBlock, 0, stream>>>(static_cast<const KEYT*>(keys), p)
-  if (key_bytes == 8) {
-    if (f16) {
-      if (vec == 16) UGC_LAUNCH_POOL(long long, true, 16); else UGC_LAUNCH_POOL(long long, true, 4);
-    } else {
-      if (vec == 16) UGC_LAUNCH_POOL(long long, false, 16); else UGC_LAUNCH_POOL(long long, false, 4);
-    }
-  } else {
-    if (f16) {
-      if (vec == 16) UGC_LAUNCH_POOL(uint32_t, true, 16); else UGC_LAUNCH_POOL(uint32_t, true, 4);
-    } else {
-      if (vec == 16) UGC_LAUNCH_POOL(uint32_t, false, 16); else UGC_LAUNCH_POOL(uint32_t, false, 4);
-    }
-  }
-#undef UGC_LAUNCH_POOL
-  return cudaGetLastError();
+  // 4-byte pieces while 16-byte ones would keep fewer than five warps an SM busy.  Few bags are bound
+  // by how many rows of one bag are in flight, many by instructions.  Measured, 4- against 16-byte:
+  // 512-byte rows, 212,992 keys in 256 bags 27.5 / 52.6 us, 512 bags 22.1 / 31.0, 1024 bags 22.0 / 19.0,
+  // 8192 bags 35.0 / 15.8; 128-byte fp16 rows, 80,000 keys in 2048 bags 8.2 / 11.2, 8192 bags 11.8 / 8.3.
+  const uint64_t lanes16 = (uint64_t)p.n_bags * (p.row_bytes / 16);
+  const int vec = vec_bytes == 4 || vec_bytes == 16 ? vec_bytes : lanes16 < (uint64_t)sm_count * 5 * 32 ? 4 : 16;
+  const int lpr = lanes_per_row(p.row_bytes, vec);
+  p.lpr_shift = 0;
+  while ((1 << p.lpr_shift) < lpr) p.lpr_shift++;
+  const uint32_t columns = (p.row_bytes / (uint32_t)vec + lpr - 1) / lpr;
+  p.col_blocks = (columns + kPoolMaxBlock / 32 - 1) / (kPoolMaxBlock / 32);
+  const uint32_t warps = (columns + p.col_blocks - 1) / p.col_blocks;
+  // bags a tile: twice the keys of a resident warp's share of the batch, and no more than the CTA's
+  // threads probe at once (104,982 keys of 32-byte rows: half of that 11.7 us, this 8.3)
+  const uint64_t avg_bag = std::max<uint64_t>(1, p.offsets ? (uint64_t)p.n_keys / p.n_bags : p.bag_size);
+  const uint64_t share = 2 * (uint64_t)p.n_keys * columns / ((uint64_t)sm_count * 32);
+  const uint64_t want = std::min<uint64_t>(std::max<uint64_t>(share, 32 / lpr), 2 * 32 * warps);
+  p.bags_per_tile = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(1, want / avg_bag), kPoolMaxBags);
+  const uint64_t grid = ((uint64_t)p.n_bags + p.bags_per_tile - 1) / p.bags_per_tile * p.col_blocks;
+  auto launch = [&](auto key, auto half, auto vec_c) {
+    using KeyT = decltype(key);
+    return launch_pdl(lookup_pool_kernel<KeyT, decltype(half)::value, decltype(vec_c)::value>, (int)grid,
+                      (int)warps * 32, 0, stream, pdl, static_cast<const KeyT*>(keys), p);
+  };
+  auto by_vec = [&](auto key, auto half) {
+    return vec == 16 ? launch(key, half, std::integral_constant<int, 16>{})
+                     : launch(key, half, std::integral_constant<int, 4>{});
+  };
+  auto by_elem = [&](auto key) { return f16 ? by_vec(key, std::true_type{}) : by_vec(key, std::false_type{}); };
+  return key_bytes == 8 ? by_elem((long long)0) : by_elem((uint32_t)0);
 }
 
 cudaError_t launch_unique_claim(const void* keys, int key_bytes, uint32_t n, uint64_t num_keys, uint32_t epoch,
