@@ -17,6 +17,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <set>
@@ -891,6 +892,8 @@ int make_stage() {
 // nid_to_block[key], looked up by the host threads on the way into the pinned staging buffer.
 // One byte instead of four crosses PCIe, at the pinned rate, and the classification reads a
 // quarter of the memory (2 M keys: 0.83 ms for the pageable block ids before, 0.1 ms now).
+// A build of up to 8 M keys does without the staging block when there is none yet: making it costs
+// 1.3 ms and giving it back 0.5, more than pageable bytes lose, and many programs never refresh.
 int upload_sources(ugc_ctx* c, Replica* r, const Placement& p, uint8_t** dst, cudaStream_t s) {
   const uint64_t N = c->cfg.num_total_item;
   if (!*dst) {
