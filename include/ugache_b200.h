@@ -349,10 +349,11 @@ int ugc_reserve_batch(ugc_ctx* ctx, int replica_id, uint32_t max_batch);
 /* Host-buffer form: keys and out are HOST pointers.  Returns after the rows have landed in
  * `out`.  key_bytes is 4 or 8.  A buffer that is pinned and mapped for the GPU (cudaHostAlloc /
  * cudaHostRegister with the mapped flag, or ugc_host_alloc) can be used in place, as
- * ugc_tuning.host_zero_copy says: by default the kernel reads the keys across PCIe itself,
- * while the rows are staged in device memory and leave through the copy engine (measured
- * faster than stores from the SMs: 56 against 51 GB/s), in four pieces for batches of 65,536
- * keys or more so that one piece crosses PCIe while the next is being extracted.  After such
+ * ugc_tuning.host_zero_copy says: by default the kernel reads the keys across PCIe itself and
+ * writes up to 4 MB of rows in place (512 KB if rows or buffer are not 32-byte aligned); more
+ * rows are staged in device memory and leave through the copy engine (measured faster than
+ * stores from the SMs: 56 against 51 GB/s), in four pieces for batches of 65,536 keys or more
+ * so that one piece crosses PCIe while the next is being extracted.  After such
  * a call ugc_stats' last_* fields describe the last piece only.  Pageable buffers always go
  * through staging copies. */
 int ugc_lookup_host(ugc_ctx* ctx, int replica_id, const void* keys, int key_bytes, size_t n,
@@ -464,7 +465,8 @@ typedef struct {
                                      groups instead of caps on the derived split (sweeps)     */
   int32_t host_zero_copy;         /* ugc_lookup_host with GPU-mapped pinned buffers: bit 0 the
                                      kernel reads the keys in place, bit 1 it writes the rows
-                                     in place; a cleared bit selects a staging copy          */
+                                     in place whatever their number (1: few rows in place);
+                                     0: staging copies                                       */
 } ugc_tuning;
 int ugc_get_tuning(ugc_ctx* ctx, int replica_id, ugc_tuning* out);
 int ugc_set_tuning(ugc_ctx* ctx, int replica_id, const ugc_tuning* in);

@@ -1,0 +1,35 @@
+"""Host-buffer lookups on both sides of the line between rows written in place and rows staged: the
+rows are copies, so they are equal or wrong, and nothing beyond them is touched."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+# 512-byte rows: 4 MB are 8192 keys; 200-byte rows, or 512-byte ones in a buffer 4 bytes off: 512 KB
+# are 2621 and 1024
+@pytest.mark.parametrize("dim,shift,ns", [(128, 0, [1, 8192, 8193]), (50, 0, [1, 2621, 2622]), (128, 4, [1, 1024, 1025])])
+@pytest.mark.parametrize("key_dtype", [np.int64, np.uint32])
+def test_host_lookup_edges(built_lib, dim, shift, ns, key_dtype):
+    from ugache_b200 import runtime as rt, workload as wl
+    N, row = 20000, dim * 4
+    table = wl.table(2, N, dim)
+    ids, freqs = wl.analytic_hotness(N, 1.1)
+    cache = rt.Cache(1, N, row, 0.5, max_batch=1 << 14)
+    cache.set_placement(rt.solve_placement("intuitive", 1, ids, freqs, 50.0))
+    host = torch.from_numpy(table).pin_memory()
+    cache.build(0, 0, host.data_ptr())
+    stream = torch.cuda.current_stream().cuda_stream
+    for n in ns:
+        keys = wl.zipf_keys(n, n, N, 1.1).astype(key_dtype)
+        k = torch.from_numpy(keys.view(np.int64 if key_dtype == np.int64 else np.int32)).pin_memory()
+        out = torch.full((shift + n * row + 64,), 7, dtype=torch.uint8).pin_memory()
+        for keys_ptr in (k.data_ptr(), keys.ctypes.data):     # pinned and pageable keys
+            out.fill_(7)
+            cache.lookup_host_ptr(0, keys_ptr, keys.itemsize, n, out.data_ptr() + shift, stream)
+            got = out.numpy()
+            assert np.array_equal(got[shift:shift + n * row].view(np.uint8).reshape(n, row),
+                                  table[keys.astype(np.int64)].view(np.uint8).reshape(n, row)), n
+            assert (got[:shift] == 7).all() and (got[shift + n * row:] == 7).all()
+    cache.close()

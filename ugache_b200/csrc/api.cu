@@ -624,7 +624,7 @@ struct Replica {
   uint64_t lookups_direct = 0;
   uint64_t kernel_launches = 0;
   uint64_t lookups_pooled = 0;
-  int host_zero_copy = 1;  // keys read in place; rows staged (the copy engine beats SM stores over PCIe)
+  int host_zero_copy = 1;  // keys read in place; rows in place when few, else staged (rows_in_place)
   // per-kernel profiling (three events per lookup)
   std::vector<cudaEvent_t> prof_events;
   size_t prof_used = 0;
@@ -904,6 +904,15 @@ int upload_sources(ugc_ctx* c, Replica* r, const Placement& p, uint8_t** dst, cu
   const uint32_t* n2b = p.nid_to_block.data();
   const int threads = std::max(1, std::min(16, omp_get_num_procs()));
   std::lock_guard<std::mutex> lock(g_stage_mu);
+  if (!r->built && !g_stage && N <= (8u << 20)) {
+    std::unique_ptr<uint8_t[]> bytes(new (std::nothrow) uint8_t[N]);
+    if (!bytes) return fail(UGC_ERR_NOMEM, "out of host memory");
+#pragma omp parallel for schedule(static) num_threads(N > 65536 ? threads : 1)
+    for (int64_t i = 0; i < (int64_t)N; i++) bytes[i] = acc[n2b[i]];
+    UGC_CUDA(cudaMemcpyAsync(*dst, bytes.get(), N, cudaMemcpyHostToDevice, s));
+    UGC_CUDA(cudaStreamSynchronize(s));
+    return UGC_OK;
+  }
   UGC_TRY(make_stage());
   int buf = 0;
   for (uint64_t off = 0; off < N; off += kStageKeys, buf = (buf + 1) % kStageParts) {
@@ -1062,6 +1071,16 @@ bool choose_direct(const Replica* r) {
   // 2376 against 2514 us with 128 k host / 317 k peer rows).
   const uint32_t host = f->count[kGroupHost], remote = f->count[kGroupRemote];
   return host <= (uint32_t)r->direct_max_host_rows || remote > host;
+}
+
+// Whether a host-buffer lookup's kernel writes the rows across PCIe itself.  A copy costs 10 us of its
+// own and starts when the last row is staged, stores from the SMs run at 51 GB/s against its 56: in
+// place while that is the smaller loss.  Measured staged / in place, us a call, 512-byte rows: 64 KB
+// 26 / 20, 1 MB 49 / 40, 4 MB 104 / 101, 8 MB 178 / 183; rows whose pieces are 4 bytes wide (200 bytes)
+// 64 KB 32 / 24, 256 KB 36 / 29, 1 MB 50 / 49, 4 MB 105 / 131.  `align`: address and row size or'ed.
+bool rows_in_place(int host_zero_copy, size_t bytes, uintptr_t align) {
+  if (host_zero_copy & 2) return true;
+  return host_zero_copy == 1 && bytes <= ((align & 31) == 0 ? (size_t)4 << 20 : (size_t)512 << 10);
 }
 
 // What the extraction of a deduplicated lookup needs besides (see DirectParams).
@@ -1934,7 +1953,13 @@ int ugc_lookup_host(ugc_ctx* c, int replica_id, const void* keys, int key_bytes,
   // Pinned buffers that the GPU has mapped are used in place: the kernel reads the keys and
   // writes the rows across PCIe itself.
   const void* keys_dev = (r->host_zero_copy & 1) ? mapped_device_pointer(keys) : nullptr;
-  void* out_dev = (r->host_zero_copy & 2) ? mapped_device_pointer(out) : nullptr;
+  const size_t rb = c->cfg.row_bytes;
+  void* out_dev = nullptr;
+  if (rows_in_place(r->host_zero_copy, n * rb, reinterpret_cast<uintptr_t>(out) | rb)) {
+    out_dev = mapped_device_pointer(out);
+    const char* last = static_cast<const char*>(out) + (n * rb - 1);  // the caller may have pinned a part
+    if (out_dev && mapped_device_pointer(last) != static_cast<char*>(out_dev) + (n * rb - 1)) out_dev = nullptr;
+  }
   if (!keys_dev) {
     UGC_TRY(ensure(c, r->stage_keys, n * (size_t)key_bytes));
     UGC_CUDA(cudaMemcpyAsync(r->stage_keys.ptr, keys, n * (size_t)key_bytes, cudaMemcpyHostToDevice, s));
@@ -1948,7 +1973,6 @@ int ugc_lookup_host(ugc_ctx* c, int replica_id, const void* keys, int key_bytes,
   // Rows are staged in device memory and leave through the copy engine, which moves them
   // faster than stores from the SMs do.  Large batches go in pieces: while piece i crosses
   // PCIe on a second stream, piece i+1 is being extracted.
-  const size_t rb = c->cfg.row_bytes;
   UGC_TRY(ensure(c, r->stage_out, n * rb));
   // four pieces, the first half the size of the others: the copy engine starts early and then
   // runs few, large copies (each copy costs about 10 us of its own)
