@@ -351,7 +351,7 @@ int ugc_reserve_batch(ugc_ctx* ctx, int replica_id, uint32_t max_batch);
  * cudaHostRegister with the mapped flag, or ugc_host_alloc) can be used in place, as
  * ugc_tuning.host_zero_copy says: by default the kernel reads the keys across PCIe itself and
  * writes up to 4 MB of rows in place (512 KB if rows or buffer are not 32-byte aligned); more
- * rows are staged in device memory and leave through the copy engine (measured faster than
+ * rows, and any rows for an address that is not a multiple of 4, are staged in device memory and leave through the copy engine (measured faster than
  * stores from the SMs: 56 against 51 GB/s), in four pieces for batches of 65,536 keys or more
  * so that one piece crosses PCIe while the next is being extracted.  After such
  * a call ugc_stats' last_* fields describe the last piece only.  Pageable buffers always go

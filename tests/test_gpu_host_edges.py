@@ -33,3 +33,26 @@ def test_host_lookup_edges(built_lib, dim, shift, ns, key_dtype):
                                   table[keys.astype(np.int64)].view(np.uint8).reshape(n, row)), n
             assert (got[:shift] == 7).all() and (got[shift + n * row:] == 7).all()
     cache.close()
+
+
+# fp16 rows at an odd element, and at odd bytes: the kernels store 4-byte words, so these are staged
+@pytest.mark.parametrize("shift", [1, 2, 3, 6])
+@pytest.mark.parametrize("zero_copy", [1, 3])
+def test_host_rows_at_any_byte(built_lib, shift, zero_copy):
+    from ugache_b200 import runtime as rt, workload as wl
+    N, dim, n = 5000, 50, 300
+    row = dim * 2
+    table = wl.table(4, N, dim, np.dtype(np.float16))
+    ids, freqs = wl.analytic_hotness(N, 1.1)
+    cache = rt.Cache(1, N, row, 0.5, max_batch=1024)
+    cache.set_placement(rt.solve_placement("intuitive", 1, ids, freqs, 50.0))
+    host = torch.from_numpy(table).pin_memory()
+    cache.build(0, 0, host.data_ptr())
+    cache.tune(0, host_zero_copy=zero_copy)
+    keys = torch.from_numpy(wl.zipf_keys(3, n, N, 1.1)).pin_memory()
+    out = torch.full((shift + n * row + 64,), 7, dtype=torch.uint8).pin_memory()
+    cache.lookup_host_ptr(0, keys.data_ptr(), 8, n, out.data_ptr() + shift, torch.cuda.current_stream().cuda_stream)
+    got = out.numpy()
+    assert got[shift:shift + n * row].tobytes() == table[keys.numpy()].tobytes()
+    assert (got[:shift] == 7).all() and (got[shift + n * row:] == 7).all()
+    cache.close()

@@ -1077,8 +1077,10 @@ bool choose_direct(const Replica* r) {
 // own and starts when the last row is staged, stores from the SMs run at 51 GB/s against its 56: in
 // place while that is the smaller loss.  Measured staged / in place, us a call, 512-byte rows: 64 KB
 // 26 / 20, 1 MB 49 / 40, 4 MB 104 / 101, 8 MB 178 / 183; rows whose pieces are 4 bytes wide (200 bytes)
-// 64 KB 32 / 24, 256 KB 36 / 29, 1 MB 50 / 49, 4 MB 105 / 131.  `align`: address and row size or'ed.
+// 64 KB 32 / 24, 256 KB 36 / 29, 1 MB 50 / 49, 4 MB 105 / 131.  `align`: address and row size or'ed;
+// the kernels store words of 4 bytes at least, so a buffer at any other address is always staged.
 bool rows_in_place(int host_zero_copy, size_t bytes, uintptr_t align) {
+  if (align & 3) return false;
   if (host_zero_copy & 2) return true;
   return host_zero_copy == 1 && bytes <= ((align & 31) == 0 ? (size_t)4 << 20 : (size_t)512 << 10);
 }
