@@ -1519,18 +1519,20 @@ int ugc_build(ugc_ctx* c, int replica_id, int device_id, const void* host_table,
   // for 208 keys, equal without host rows).
   r->vec_bytes = c->cfg.gather_vec_bytes ? (c->cfg.gather_vec_bytes == 32 ? 32 : 16) : (G >= 8 ? 32 : 16);
 
+  // a build that fails gives everything back once the stream is done with it: a caller's allocator
+  // may hand the memory on at once
+  auto bail = [&](int rc) {
+    std::string keep = g_last_error;
+    cudaStreamSynchronize(s);
+    release_replica(c, r);
+    g_last_error = keep;
+    return rc;
+  };
+  int rc;
   // 1. which source serves each key: ascending key lists per GPU source, made on the GPU
-  {
-    int rc0 = make_pinned(r);
-    if (rc0 == UGC_OK) rc0 = upload_sources(c, r, c->cur, &r->src_dev, s);
-    if (rc0 == UGC_OK) rc0 = gpu_classify(c, r, nullptr, r->src_dev, s);
-    if (rc0 != UGC_OK) {
-      std::string keep = g_last_error;
-      release_replica(c, r);
-      g_last_error = keep;
-      return rc0;
-    }
-  }
+  if ((rc = make_pinned(r)) != UGC_OK) return bail(rc);
+  if ((rc = upload_sources(c, r, c->cur, &r->src_dev, s)) != UGC_OK) return bail(rc);
+  if ((rc = gpu_classify(c, r, nullptr, r->src_dev, s)) != UGC_OK) return bail(rc);
   const uint64_t n_local = r->list_count[replica_id];
   uint64_t n_remote = 0;
   for (int s2 = 0; s2 < G; s2++)
@@ -1540,26 +1542,12 @@ int ugc_build(ugc_ctx* c, int replica_id, int device_id, const void* host_table,
 
   // 2. the slice
   r->capacity = cache_capacity_rows(N, c->cfg.cache_percentage);
-  if (n_local > r->capacity) {
-    int rc = fail(UGC_ERR_CAPACITY, "placement stores %llu rows on replica %d, slice holds %llu",
-                  (unsigned long long)n_local, replica_id, (unsigned long long)r->capacity);
-    release_replica(c, r);
-    return rc;
-  }
+  if (n_local > r->capacity)
+    return bail(fail(UGC_ERR_CAPACITY, "placement stores %llu rows on replica %d, slice holds %llu",
+                     (unsigned long long)n_local, replica_id, (unsigned long long)r->capacity));
   r->slice_bytes = std::max<size_t>((size_t)r->capacity * c->cfg.row_bytes, 256);
   r->slice = ctx_alloc_shared(c, r->slice_bytes);
-  if (!r->slice) {
-    int rc = fail(UGC_ERR_NOMEM, "slice allocation of %zu bytes failed", r->slice_bytes);
-    release_replica(c, r);
-    return rc;
-  }
-  auto bail = [&](int rc) {
-    std::string keep = g_last_error;
-    release_replica(c, r);
-    g_last_error = keep;
-    return rc;
-  };
-  int rc;
+  if (!r->slice) return bail(fail(UGC_ERR_NOMEM, "slice allocation of %zu bytes failed", r->slice_bytes));
   // 3. lookup scratch and counters
   if ((rc = make_scratch(c, &r->scratch, c->cfg.max_batch, s)) != UGC_OK) return bail(rc);
   use_scratch(r, c->cfg.max_batch);
@@ -2037,8 +2025,10 @@ int ugc_refresh_evict(ugc_ctx* c, int replica_id, void* stream) {
   const uint64_t n_evict = r->list_count[kListEvict], n_insert = r->list_count[kListInsert];
   const uint64_t n_drop = r->list_count[kListDropRemote];
   const uint64_t n_new_local = r->n_local - n_evict + n_insert;
-  // a placement that does not fit is refused before anything changed
+  // a placement that does not fit is refused before anything changed; the lists are still being
+  // written, and the next refresh may classify on another stream or a caller's allocator reuse them
   auto refuse = [&](int rc) {
+    UGC_CUDA(cudaStreamSynchronize(s));
     release_lists(c, r);
     return rc;
   };
