@@ -313,7 +313,8 @@ int ugc_lookup_i64_static(ugc_ctx* ctx, int replica_id, const int64_t* keys, siz
  *                                synchronises; capacity of out_rows / unique_keys: n entries.
  * keys: key_bytes 4 or 8.  Uses one 32-bit stamp per id of the key space (allocated on the
  * first call); at most 2^24-2 keys per call.  After the call ugc_stats' last_local/remote/host
- * add up to the number of distinct keys.  The reference has no such call; its applications
+ * add up to the number of distinct keys.  May be captured into a graph once a first call has run;
+ * the graph then clears the stamps itself.  The reference has no such call; its applications
  * deduplicate before they look up (example/dlr and the GNN samplers hand over unique ids). */
 int ugc_lookup_unique(ugc_ctx* ctx, int replica_id, const void* keys, int key_bytes, size_t n,
                       void* out_rows, void* unique_keys, int32_t* inverse, uint32_t* n_unique,

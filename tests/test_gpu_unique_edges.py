@@ -36,3 +36,50 @@ def test_unique_edges(built_lib, n, spread):
         assert torch.equal(rows.view(torch.float32)[:nu][inverse.long()], rows_of[k])
         assert torch.equal(again, rows_of[inverse.long()])
     cache.close()
+
+
+def test_capture_between_calls(built_lib):
+    """Calls captured into graphs -- never launched, launched once, launched again on other keys -- and
+    ordinary calls between them, over the turn of the epochs."""
+    from ugache_b200 import runtime as rt, workload as wl
+    N, dim, n = 50_000, 4, 3000
+    table = wl.table(6, N, dim)
+    ids, freqs = wl.analytic_hotness(N, 1.2)
+    cache = rt.Cache(1, N, dim * 4, 0.5, max_batch=n)
+    cache.set_placement(rt.solve_placement("intuitive", 1, ids, freqs, 50.0))
+    host = torch.from_numpy(table).pin_memory()
+    cache.build(0, 0, host.data_ptr())
+    rows_of = torch.from_numpy(table).cuda()
+    r = np.random.default_rng(3)
+    draw = lambda: torch.from_numpy(r.integers(0, N, n)).cuda()
+
+    def check(result, k):
+        rows, uniq, inverse, n_unique = result
+        nu = int(n_unique)
+        assert nu == int(torch.unique(k).numel())
+        assert int(inverse.min()) >= 0 and int(inverse.max()) < nu
+        assert torch.equal(uniq[:nu][inverse.long()], k)
+        assert torch.equal(rows.view(torch.float32)[:nu][inverse.long()], rows_of[k])
+
+    def eager():
+        k = draw()
+        check(cache.lookup_unique(0, k), k)
+
+    eager()
+    static = draw()
+    graphs = []
+    for _ in range(90):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            result = cache.lookup_unique(0, static)
+        graphs.append((g, result))
+        eager()                          # the captured call has not run
+        for g, result in graphs[-2:]:
+            for _ in range(2):
+                static.copy_(draw())
+                g.replay()
+                check(result, static)
+        eager()
+        if len(graphs) > 3:
+            graphs.pop(0)
+    cache.close()

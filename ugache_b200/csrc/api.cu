@@ -579,6 +579,7 @@ struct Replica {
   uint32_t* stamp = nullptr;               // deduplicated lookups: one stamp per id (first use)
   uint32_t stamp_epoch = 0;
   uint32_t unique_slot = 0;                // which of Counters::unique_count the next one uses
+  bool unique_dirty = false;               // a call failed between its launches: the slots hold rests
   int host_order_min_rows = 8192;
   uint64_t lookups_host_ordered = 0;
   uint32_t direct_slot = 0, last_slot = 0; // count slot of the next / the last direct launch
@@ -1090,7 +1091,7 @@ struct UniqueArgs {
   const void* batch_keys;
   int32_t* inverse;
   uint32_t* n_unique;
-  uint32_t slot;
+  uint32_t slot, clear;
 };
 
 // `uniq` != nullptr: `keys` are the distinct ones of a batch of n, left by the claim just ahead in the
@@ -1116,6 +1117,7 @@ int do_lookup(ugc_ctx* c, Replica* r, const void* keys, int key_bytes, size_t n,
       d.inverse = uniq->inverse;
       d.n_unique = uniq->n_unique;
       d.unique_slot = uniq->slot;
+      d.unique_clear = uniq->clear;
     }
     for (int i = 0; i < kMaxLocation; i++) d.src_base[i] = r->src_base[i];
     d.out = out;
@@ -1824,6 +1826,9 @@ int ugc_lookup_i64_static(ugc_ctx* c, int replica_id, const int64_t* keys, size_
   return UGC_OK;
 }
 
+// Epochs of deduplicated lookups: 1 .. kLastEpoch in turn, the one after it for captured calls.
+static constexpr uint32_t kLastEpoch = 254;
+
 int ugc_lookup_unique(ugc_ctx* c, int replica_id, const void* keys, int key_bytes, size_t n, void* out_rows,
                       void* unique_keys, int32_t* inverse, uint32_t* n_unique, void* stream) {
   Replica* r;
@@ -1845,18 +1850,38 @@ int ugc_lookup_unique(ugc_ctx* c, int replica_id, const void* keys, int key_byte
   if (!r->stamp) {
     r->stamp = static_cast<uint32_t*>(ctx_alloc(c, stamp_bytes));
     if (!r->stamp) return fail(UGC_ERR_NOMEM, "stamp array (%zu bytes) could not be allocated", stamp_bytes);
-    r->stamp_epoch = 255;  // forces the clearing below
+    r->stamp_epoch = kLastEpoch;  // forces the clearing below
   }
-  if (++r->stamp_epoch > 255) {  // all stamps back to epoch 0 before an epoch value is reused
+  // A captured call runs as often as its graph is launched, in any order with other calls, so it takes
+  // nothing from the host's sequence of epochs and slots: an epoch and a slot of its own, both cleared
+  // by the graph itself.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+  const bool captured = cap == cudaStreamCaptureStatusActive;
+  uint32_t* counts = r->counters->unique_count;
+  uint32_t epoch = kLastEpoch + 1;
+  UniqueArgs uniq{keys, inverse, n_unique, 2, kNoSlot};
+  if (captured) {
     UGC_CUDA(cudaMemsetAsync(r->stamp, 0, stamp_bytes, s));
-    r->stamp_epoch = 1;
+    UGC_CUDA(cudaMemsetAsync(counts + uniq.slot, 0, sizeof(uint32_t), s));
+  } else {
+    if (++r->stamp_epoch > kLastEpoch) {  // all stamps back to epoch 0 before an epoch value is reused
+      UGC_CUDA(cudaMemsetAsync(r->stamp, 0, stamp_bytes, s));
+      r->stamp_epoch = 1;
+    }
+    if (r->unique_dirty) UGC_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(uint32_t), s));
+    epoch = r->stamp_epoch;
+    uniq.slot = r->unique_slot;
+    uniq.clear = uniq.slot ^ 1u;
+    r->unique_slot ^= 1u;
+    r->unique_dirty = true;  // until the extraction, which clears the next slot, is on its way
   }
-  const UniqueArgs uniq{keys, inverse, n_unique, r->unique_slot};
-  UGC_CUDA(launch_unique_claim(keys, key_bytes, (uint32_t)n, c->cfg.num_total_item, r->stamp_epoch, r->stamp,
-                               unique_keys, &r->counters->unique_count[uniq.slot], r->counters, (r->pdl & 1) != 0, s));
-  r->unique_slot ^= 1u;
+  UGC_CUDA(launch_unique_claim(keys, key_bytes, (uint32_t)n, c->cfg.num_total_item, epoch, r->stamp, unique_keys,
+                               counts + uniq.slot, r->counters, (r->pdl & 1) != 0, s));
   r->kernel_launches += 1;
-  return do_lookup(c, r, unique_keys, key_bytes, n, out_rows, s, &uniq);
+  UGC_TRY(do_lookup(c, r, unique_keys, key_bytes, n, out_rows, s, &uniq));
+  if (!captured) r->unique_dirty = false;
+  return UGC_OK;
 }
 
 int ugc_lookup_pool(ugc_ctx* c, int replica_id, const void* keys, int key_bytes, size_t n_keys,

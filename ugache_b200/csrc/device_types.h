@@ -74,8 +74,9 @@ struct Counters {
   // direct extraction: per-source counts of the launches that own slot 0 / slot 1 in turn; a
   // launch adds to its slot and clears the other one (whose launch is complete by then)
   uint32_t dcount[2][kNumGroup];
-  // deduplicated lookups: distinct keys found, in slots used in turn like dcount's
-  uint32_t unique_count[2];
+  // deduplicated lookups: distinct keys found.  Slots 0 and 1 are used in turn like dcount's; slot 2
+  // is that of captured calls, which bring their own clearing
+  uint32_t unique_count[3];
   alignas(16) uint32_t shown[kNumGroup + 1];  // what the pinned mirror shows: counts and ordinal
   // pooled lookups: rows summed so far, per source group (cumulative)
   unsigned long long pool_rows[kNumGroup];
@@ -135,6 +136,7 @@ struct PoolParams {
 };
 
 // Everything the direct extraction (lookup and row copy in one kernel, no index lists) needs.
+constexpr uint32_t kNoSlot = 0xffffffffu;
 struct DirectParams {
   const void* src_base[kMaxLocation];
   void* out;
@@ -148,6 +150,7 @@ struct DirectParams {
   int32_t* inverse;     // out: index of every key of the batch, -1 for an id outside the table
   uint32_t* n_unique;   // out: number of distinct keys
   uint32_t unique_slot;
+  uint32_t unique_clear;  // the slot to clear for the next deduplicated lookup; kNoSlot: none
   const void* host_base;  // src_base[host_loc], for the kernel's prologue
   uint32_t n_keys;
   uint32_t row_bytes;

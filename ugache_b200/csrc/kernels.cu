@@ -1057,7 +1057,7 @@ __global__ void __launch_bounds__(kBlock, DEEP ? 3 : 4)
       p.counters->last_keys = p.n_keys;
       if (UNIQUE) {
         *p.n_unique = n_keys;
-        p.counters->unique_count[p.unique_slot ^ 1u] = 0;  // for the next deduplicated lookup
+        if (p.unique_clear != kNoSlot) p.counters->unique_count[p.unique_clear] = 0;  // for the next one
       }
     }
   };
