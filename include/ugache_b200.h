@@ -274,7 +274,12 @@ int ugc_attach_peers(ugc_ctx* ctx, int replica_id, void* stream);
  * streams are idle; its shim adds the synchronise).  Replaces CollCache::lookup ->
  * ExtractSession::ExtractFeat (coll_cache_lib/facade.cc:74-88,
  * coll_cache_lib/cache_context.cu:1199) and coll_cache_lookup
- * (python/collcache/common/operation.cc:232-236), whose keys are 32-bit. */
+ * (python/collcache/common/operation.cc:232-236), whose keys are 32-bit.
+ * Ordered on the stream like any other work: keys, table rows and `out` may come from whatever was
+ * enqueued before, another lookup's rows among it.  Only a kernel of the caller's that is itself
+ * launched with programmatic stream serialization and releases its dependents ahead of its own
+ * dependency wait must not write what the lookup behind it reads (or switch
+ * ugc_tuning.programmatic_launch off). */
 int ugc_lookup_u32(ugc_ctx* ctx, int replica_id, const uint32_t* keys, size_t n, void* out,
                    void* stream);
 /* Same with 64-bit ids (results identical for ids below 2^31-1). */
@@ -424,7 +429,8 @@ typedef struct {
   int32_t lookup_keys_per_thread; /* 1, 2 or 4; 0 (default) = chosen by the batch size       */
   int32_t programmatic_launch;    /* programmatic stream serialization: bit 0 for the lookup
                                      kernel (its key loads and probes overlap the tail of
-                                     the previous gather), bit 1 for the gather kernel (it is
+                                     the previous gather) and for deduplicated and pooled
+                                     lookups, bit 1 for the gather kernel (it is
                                      scheduled while the lookup kernel drains)              */
   int32_t extract_mode;           /* ugc_extract_mode                                       */
   int32_t direct_ctas_per_sm;     /* CTAs of the direct extraction kernel per SM, 1..16     */

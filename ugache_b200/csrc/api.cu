@@ -996,7 +996,6 @@ GatherParams gather_params(ugc_ctx* c, Replica* r, void* out, uint32_t n) {
   p.host_cta_cap = r->host_ctas;
   p.rows_per_cta_min = 32;
   for (int g = 0; g < kNumGroup; g++) p.t_byte[g] = r->t_byte[g];
-  p.seq = (uint32_t)r->lookups;
   p.dynamic = r->gather_dynamic;
   p.fixed_split = r->split_fixed;
   p.bulk_mask = r->bulk_mask;
@@ -1094,6 +1093,82 @@ struct UniqueArgs {
   uint32_t slot, clear;
 };
 
+// What tells the streams of lookups apart: the driver's entry points, since the runtime's wrappers took
+// four times as long (75 against 24 ns of a 4.5 us call).
+struct StreamApi {
+  CUresult (*capture_info)(CUstream, CUstreamCaptureStatus*, cuuint64_t*, CUgraph*, const CUgraphNode**, size_t*) = nullptr;
+  CUresult (*get_id)(CUstream, unsigned long long*) = nullptr;
+};
+const StreamApi& stream_api() {
+  static const StreamApi api = [] {
+    StreamApi a;
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult st;
+    if (cudaGetDriverEntryPointByVersion("cuStreamGetCaptureInfo", &fn, 11030, cudaEnableDefault, &st) == cudaSuccess &&
+        st == cudaDriverEntryPointSuccess)
+      a.capture_info = reinterpret_cast<decltype(a.capture_info)>(fn);
+    if (cudaGetDriverEntryPointByVersion("cuStreamGetId", &fn, 12000, cudaEnableDefault, &st) == cudaSuccess &&
+        st == cudaDriverEntryPointSuccess)
+      a.get_id = reinterpret_cast<decltype(a.get_id)>(fn);
+    cudaGetLastError();
+    return a;
+  }();
+  return api;
+}
+
+// The extraction enqueued last on a stream, of whatever cache; streams share the kRunSlots entries by hash.
+struct LastExtraction {
+  int device = -1;
+  unsigned long long stream = 0;    // id of the stream (a handle may come back, or stand for one stream per
+  cudaStream_t captured = nullptr;  // thread); in a capture, where it cannot be asked for, capture and handle
+  uint32_t seq = 0;
+  uint32_t marks = 0;
+  uintptr_t out = 0, end = 0;  // what it writes
+};
+std::mutex g_order_mu;
+LastExtraction g_last[kRunSlots];
+uint32_t g_extractions = 0;
+
+// Place of the extraction being enqueued in its stream.  It may read past the one ahead (order.ahead) unless
+// that one's output holds its keys or its host table.  Other threads may enqueue in any order meanwhile:
+// the ordinal of an extraction that is not the one right ahead is no longer, or not yet, among the marks.
+StreamOrder order_in_stream(ugc_ctx* c, Replica* r, const void* keys, size_t key_bytes, const void* out,
+                            size_t out_bytes, bool direct, cudaStream_t s) {
+  const StreamApi& api = stream_api();
+  LastExtraction me;
+  cuuint64_t capture_id = 0;
+  CUstreamCaptureStatus cap = CU_STREAM_CAPTURE_STATUS_NONE;
+  bool known = api.capture_info && api.get_id &&
+               api.capture_info(s, &cap, &capture_id, nullptr, nullptr, nullptr) == CUDA_SUCCESS;
+  if (cap != CU_STREAM_CAPTURE_STATUS_NONE) {
+    me.stream = capture_id;
+    me.captured = s;
+  } else if (known) {
+    known = api.get_id(s, &me.stream) == CUDA_SUCCESS;
+  }
+  StreamOrder o{};
+  if (!known || !(r->pdl & 1)) return o;
+  me.device = r->device;
+  me.marks = direct ? kRunMarks : 1;
+  me.out = reinterpret_cast<uintptr_t>(out);
+  me.end = me.out + out_bytes;
+  o.slot = (uint32_t)((me.stream + (reinterpret_cast<uintptr_t>(me.captured) >> 4)) % kRunSlots);
+  const uint64_t host_rows = c->cfg.empty_feat > 0 ? ((uint64_t)1 << c->cfg.empty_feat) : c->cfg.num_total_item;
+  std::lock_guard<std::mutex> lock(g_order_mu);
+  LastExtraction& last = g_last[o.slot];
+  auto apart = [&](const void* p, size_t bytes) {
+    const uintptr_t lo = reinterpret_cast<uintptr_t>(p);
+    return lo + bytes <= last.out || lo >= last.end;
+  };
+  if (last.device == me.device && last.stream == me.stream && last.captured == me.captured && apart(keys, key_bytes) &&
+      apart(c->host_dev, (size_t)host_rows * c->cfg.row_bytes))
+    o.ahead = last.seq, o.marks = last.marks;
+  if (++g_extractions == 0) g_extractions = 1;
+  o.seq = me.seq = g_extractions;
+  last = me;
+  return o;
+}
+
 // `uniq` != nullptr: `keys` are the distinct ones of a batch of n, left by the claim just ahead in the
 // stream together with their number; such a lookup always takes the direct extraction.
 int do_lookup(ugc_ctx* c, Replica* r, const void* keys, int key_bytes, size_t n, void* out,
@@ -1107,8 +1182,11 @@ int do_lookup(ugc_ctx* c, Replica* r, const void* keys, int key_bytes, size_t n,
   const bool prof = r->prof_on && r->prof_used + 3 <= r->prof_events.size();
   if (prof) UGC_CUDA(cudaEventRecord(r->prof_events[r->prof_used], s));
   // counted before the launch: drain_lookups() must never miss a lookup that could be running
-  __atomic_fetch_add(&r->lookups, 1, __ATOMIC_SEQ_CST);
-  if (uniq != nullptr || choose_direct(r)) {
+  const uint32_t seq = (uint32_t)__atomic_add_fetch(&r->lookups, 1, __ATOMIC_SEQ_CST);
+  const bool direct = uniq != nullptr || choose_direct(r);
+  const StreamOrder order =
+      order_in_stream(c, r, keys, n * (size_t)key_bytes, out, n * (size_t)c->cfg.row_bytes, direct, s);
+  if (direct) {
     if (prof) UGC_CUDA(cudaEventRecord(r->prof_events[r->prof_used + 1], s));
     DirectParams d{};
     if (uniq) {
@@ -1133,6 +1211,7 @@ int do_lookup(ugc_ctx* c, Replica* r, const void* keys, int key_bytes, size_t n,
     // count slots alternate from one direct launch to the next; a launch also hands on the
     // counts of the direct launch before it
     d.slot = r->direct_slot;
+    d.order = order;
     d.publish_prev = r->last_was_direct ? 1u : 0u;
     d.prev_seq = r->last_seq;
     r->direct_slot ^= 1u;
@@ -1164,10 +1243,12 @@ int do_lookup(ugc_ctx* c, Replica* r, const void* keys, int key_bytes, size_t n,
   const uint64_t host_rows = c->cfg.empty_feat > 0 ? ((uint64_t)1 << c->cfg.empty_feat) : c->cfg.num_total_item;
   UGC_CUDA(launch_lookup_group(keys, key_bytes, (uint32_t)n, r->table, (uint32_t)r->id,
                                (uint32_t)c->cfg.num_device, c->cfg.empty_feat, r->list[kGroupLocal],
-                               r->list[kGroupRemote], r->list[kGroupHost], r->counters, r->lookup_kpt, hist, host_rows,
+                               r->list[kGroupRemote], r->list[kGroupHost], r->counters, order, r->lookup_kpt, hist, host_rows,
                                (r->pdl & 1) != 0, s));
   if (prof) UGC_CUDA(cudaEventRecord(r->prof_events[r->prof_used + 1], s));
   GatherParams p = gather_params(c, r, out, (uint32_t)n);
+  p.seq = seq;
+  p.order = order;
   if (hist) {
     UGC_CUDA(launch_host_order(r->list[kGroupHost], r->host_sorted, r->counters, hist, host_rows, r->sm_count,
                                (r->pdl & 2) != 0, s));
@@ -1807,7 +1888,7 @@ int ugc_lookup_i64_static(ugc_ctx* c, int replica_id, const int64_t* keys, size_
   UGC_CUDA(cudaMemsetAsync(counters, 0, sizeof(Counters), s));
   UGC_CUDA(launch_lookup_group(keys, 8, (uint32_t)n, r->table, (uint32_t)r->id, (uint32_t)c->cfg.num_device,
                                c->cfg.empty_feat, lists, lists + kStaticMaxKeys, lists + 2 * (size_t)kStaticMaxKeys,
-                               counters, r->lookup_kpt, nullptr, 0, false, s));
+                               counters, StreamOrder{}, r->lookup_kpt, nullptr, 0, false, s));
   GatherParams p{};
   for (int i = 0; i < kMaxLocation; i++) p.src_base[i] = r->src_base[i];
   p.out = out;

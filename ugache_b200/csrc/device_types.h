@@ -82,6 +82,16 @@ struct Counters {
   unsigned long long pool_rows[kNumGroup];
 };
 
+// How a launch tells that the extraction ahead of it in its stream still runs (see still_running).
+constexpr int kRunMarks = 128;  // CTAs that announce themselves, of the 592 of a large direct extraction
+constexpr int kRunSlots = 64;   // streams, by hash
+struct StreamOrder {
+  uint32_t slot;   // the stream's marks
+  uint32_t seq;    // this extraction's ordinal in the process; 0: not announced
+  uint32_t ahead;  // that of the extraction ahead, past which keys, table and rows may be read; 0: none
+  uint32_t marks;  // how many of its marks that one uses
+};
+
 // Written by an extraction into pinned host memory when its counts have moved: the host reads it
 // without synchronising to pick the extraction mode of the lookups it enqueues next.
 struct alignas(16) Feedback {
@@ -108,6 +118,7 @@ struct GatherParams {
   // to rows * row_bytes * t_byte of the groups, within the caps above.
   float t_byte[kNumGroup];
   uint32_t seq;         // ordinal of this lookup among the replica's lookups (for the mirror)
+  StreamOrder order;
   int dynamic;          // 1: lists are handed out in chunks; a CTA whose own list is drained
                         //    takes chunks of the other groups' lists.  0: fixed striding.
   int pdl;              // launched with programmatic stream serialization
@@ -160,6 +171,7 @@ struct DirectParams {
   uint32_t lpr_shift;   // log2 of the lanes that share one row
   uint32_t tile_shift;  // log2 of the keys one warp probes at a time; above 5: the kernel chooses
   uint32_t slot;        // which of Counters::dcount this launch adds to (launches alternate)
+  StreamOrder order;
   uint32_t publish_prev;  // 1: the launch before this one was a direct one; hand its counts on
   uint32_t prev_seq;      // its ordinal among the replica's lookups
 };

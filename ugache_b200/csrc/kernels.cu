@@ -162,6 +162,47 @@ __device__ __forceinline__ uint32_t table_lookup(const TableView& t, uint32_t ke
   return probe_rest(t.slots, t.line_mask, key, line);
 }
 
+// Keys: read once, and past the L1, which other launches of the stream overlap with.  Volatile, so that
+// they stay on their side of the dependency wait.
+__device__ __forceinline__ uint64_t ld_key(const uint32_t* p) {
+  uint32_t k;
+  asm volatile("ld.global.cg.b32 %0, [%1];" : "=r"(k) : "l"(p) : "memory");
+  return k;
+}
+__device__ __forceinline__ uint64_t ld_key(const long long* p) {
+  uint64_t k;
+  asm volatile("ld.global.cg.b64 %0, [%1];" : "=l"(k) : "l"(p) : "memory");
+  return k;
+}
+
+// Extractions that run, by stream: CTA i < kRunMarks puts the extraction's ordinal into mark i once it is
+// past its dependency wait and takes it out when it ends (the grouped gather: mark 0, for the whole grid).
+__device__ __align__(128) uint32_t g_running[kRunSlots][kRunMarks];
+
+// Whether the extraction ahead still runs.  Only then may a launch read keys, table and rows ahead of its
+// dependency wait: it has nothing but that extraction to wait for.  All that came before is complete, since
+// the extraction was past its own wait; no ordinary kernel or copy stands in between, which would have
+// waited for the extraction's end; and the library's other kernels let the next launch start no earlier
+// than behind their wait.  What the extraction ahead writes itself, its rows, the host keeps apart
+// (order_in_stream).  Without this proof a launch waits first.  Waiting first always costs 13,312 keys back
+// to back 2.0 us of 6.5, and 212,992 keys with 7,277 host rows 15 of 102.  The marks are read once a CTA, and
+// no more of them than in use: the same line read by every warp cost 500,009 keys 5 to 10 us of 164, 128 marks
+// a CTA 3.  With 8 marks of a direct extraction instead of 128 its last CTAs, which wait for host rows, were
+// missed (100 M x 512-byte rows, 3,217 host rows: 89.4 us, with 128 87.7).  All threads of the CTA take part.
+__device__ __forceinline__ bool still_running(const StreamOrder& o) {
+  if (o.ahead == 0) return false;
+  uint32_t mark = 0;
+  if (threadIdx.x < o.marks)
+    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(mark) : "l"(&g_running[o.slot][threadIdx.x]) : "memory");
+  return __syncthreads_or(mark == o.ahead);
+}
+__device__ __forceinline__ void set_running(const StreamOrder& o, uint32_t mark) {
+  if (o.seq) *const_cast<volatile uint32_t*>(&g_running[o.slot][mark]) = o.seq;
+}
+__device__ __forceinline__ void clear_running(const StreamOrder& o, uint32_t mark) {
+  if (o.seq) asm volatile("red.relaxed.gpu.global.and.b32 [%0], %1;" ::"l"(&g_running[o.slot][mark]), "r"(0u) : "memory");
+}
+
 // Address range of a host row, for the ordering of the host list.
 constexpr int kHostBuckets = 4096;
 __device__ __forceinline__ uint32_t host_bucket(uint32_t off, uint32_t shift) {
@@ -179,7 +220,7 @@ __global__ void __launch_bounds__(kBlock)
     lookup_group_kernel(const KeyT* __restrict__ keys, uint32_t n, TableView t, uint32_t local_loc,
                         uint32_t host_loc, uint32_t host_mask, uint64_t* __restrict__ list_local,
                         uint64_t* __restrict__ list_remote, uint64_t* __restrict__ list_host,
-                        Counters* counters, uint32_t* host_hist, uint32_t hist_shift) {
+                        Counters* counters, StreamOrder order, uint32_t* host_hist, uint32_t hist_shift) {
   __shared__ uint32_t s_cnt[kWarpsPerBlock][kKeysPerThread][kNumGroup];
   __shared__ uint32_t s_base[kNumGroup];
 
@@ -189,6 +230,7 @@ __global__ void __launch_bounds__(kBlock)
   unsigned long long t_begin = 0;
   if (blockIdx.x == 0 && tid == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_begin));
 
+  if (!still_running(order)) asm volatile("griddepcontrol.wait;" ::: "memory");
   uint32_t key[kKeysPerThread];
   bool valid[kKeysPerThread];
   uint32_t bad = 0;
@@ -196,7 +238,7 @@ __global__ void __launch_bounds__(kBlock)
   for (int j = 0; j < kKeysPerThread; j++) {
     uint32_t idx = tile_base + j * kBlock + tid;
     valid[j] = idx < n;
-    uint64_t k = valid[j] ? (uint64_t)keys[idx] : 0;
+    uint64_t k = valid[j] ? ld_key(keys + idx) : 0;
     if (k >= t.num_keys) {  // also catches negative int64 ids
       valid[j] = false;
       bad++;
@@ -238,9 +280,9 @@ __global__ void __launch_bounds__(kBlock)
     }
   }
 
-  // Keys and table have been read; everything below touches the lists and counters that
-  // the previous lookup's gather may still be using: wait for it (no-op unless this kernel
-  // was launched with programmatic stream serialization).
+  // Everything below touches the lists and counters that the previous lookup's gather may still
+  // be using: wait for it (no-op unless this kernel was launched with programmatic stream
+  // serialization, and if it has waited already).
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (bad) atomicAdd(&counters->err_key_range, (unsigned long long)bad);
   if (blockIdx.x == 0 && tid < kNumGroup) counters->t_end[tid] = 0;  // re-armed for the gather's timestamps
@@ -540,6 +582,7 @@ __global__ void __launch_bounds__(1024) gather_roles_kernel(GatherParams p) {
   const int b = (int)blockIdx.x;
   // The lookup kernel ahead of this one in the stream must have finished writing the lists.
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (b == 0 && threadIdx.x == 0) set_running(p.order, 0);
   // The next lookup's key loads and table probes may start while this grid drains.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   unsigned long long t0 = 0;
@@ -684,6 +727,7 @@ __global__ void __launch_bounds__(1024) gather_roles_kernel(GatherParams p) {
 #pragma unroll
       for (int g2 = 0; g2 < kNumGroup; g2++) p.counters->cursor[g2] = 0;
       publish_feedback(p.feedback, p.counters, cnt, p.seq);
+      clear_running(p.order, 0);
       __threadfence();
     }
   }
@@ -920,7 +964,7 @@ __device__ __forceinline__ void fetch_key(const KeyT* __restrict__ keys, uint32_
                                           uint32_t lane, uint32_t& key, bool& valid, uint32_t& bad) {
   const uint32_t idx = (tl << shift) + lane;
   valid = tl < n_tiles && (lane >> shift) == 0 && idx < n_keys;
-  uint64_t k = valid ? (uint64_t)keys[idx] : 0;
+  uint64_t k = valid ? ld_key(keys + idx) : 0;
   if (k >= num_keys) {  // also catches negative int64 ids
     valid = false;
     bad++;
@@ -986,51 +1030,21 @@ __global__ void __launch_bounds__(kBlock, DEEP ? 3 : 4)
 
   uint32_t bad = 0;
 
-  // Keys and table are not written by the extraction ahead of this one in the stream: the
-  // first two key loads and the first probe run before the dependency wait.
-  uint32_t key_cur, key_nxt;
-  bool ok_cur, ok_nxt;
-  fetch_key(keys, tile, n_tiles, tshift, n_keys, p.table.num_keys, lane, key_cur, ok_cur, bad);
-  fetch_key(keys, tile + n_warps, n_tiles, tshift, n_keys, p.table.num_keys, lane, key_nxt, ok_nxt, bad);
-  Probe<FLAT> pr;
-  probe_issue(p.table, key_cur, ok_cur, pr);
-  if (!UNIQUE) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  auto batch_index = [&](uint64_t k) {  // index of an id of the batch among the distinct ones
-    return k < p.table.num_keys ? (int32_t)(__ldcg(p.stamp + k) & kStampPending) : -1;
-  };
-  int32_t inv_idx[2];
-  if (UNIQUE) {
-#pragma unroll
-    for (int j = 0; j < 2; j++) inv_idx[j] = batch_index(inv_key[j]);
-  }
-  uint32_t word = probe_resolve(p.table, pr, key_cur, ok_cur);
-  // EARLY: the first host row of this warp's first tile is fetched before the dependency wait
-  // (the host table is never written by a lookup) and held in registers, one piece per lane.
-  // CTAs of this launch become resident while the launch ahead is still waiting for ITS last
-  // host rows; their requests keep the host link's queue filled across the boundary between
-  // two launches, where it would otherwise run empty and fill up again.
-  Vec<VEC> early;
-  uint32_t early_lane = 32;  // lane whose key the held row belongs to; 32 = none
-  if (EARLY) {
-    const bool is_host = ok_cur && word == kEmptyWord;
-    const unsigned hmask = __ballot_sync(kFull, is_host);
-    if (hmask && p.row_bytes / VEC <= 32) {
-      early_lane = __ffs(hmask) - 1;
-      const uint32_t k = __shfl_sync(kFull, key_cur, early_lane);
-      if (lane < p.row_bytes / VEC)
-        ld_row(early, static_cast<const char*>(p.host_base) + (size_t)(k & p.host_mask) * p.row_bytes +
-                          (size_t)lane * VEC);
-    }
-  }
-  // The dependency wait itself comes as late as it can: behind the loads of this warp's first rows,
-  // which no extraction writes either, and ahead of its first store (the batch ahead may have had
-  // the same output buffer).  A batch of one pass per warp then has all its loads behind it when
-  // the launch ahead ends (208 keys back to back: 4.3 -> 2.6 us, one key 2.4 -> 1.3).
+  // The dependency wait comes first, unless the extraction ahead still runs (still_running): then the
+  // first two key loads and the first probe go out ahead of it.
   bool waited = false;
-  const uint32_t early_tile = tile, early_row = early_lane;
+  Vec<VEC> early;
+  uint32_t early_row = 32;  // lane whose key the row in `early` belongs to; 32 = none
+  const uint32_t early_tile = tile;
   auto wait_for_launch_ahead = [&]() {
     waited = true;
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!UNIQUE) {
+      // The next launch may start: behind the wait, so that whatever it finds running or waits for,
+      // nothing older than this extraction is still under way.
+      if (blockIdx.x < kRunMarks && lane == 0) set_running(p.order, blockIdx.x);
+      asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     if (EARLY && early_row < 32) {
       if (lane < p.row_bytes / VEC)
         st_row(static_cast<char*>(p.out) + (((size_t)early_tile << tshift) + early_row) * p.row_bytes +
@@ -1061,6 +1075,45 @@ __global__ void __launch_bounds__(kBlock, DEEP ? 3 : 4)
       }
     }
   };
+  const bool ahead_runs = !UNIQUE && still_running(p.order);
+  if (!UNIQUE && !ahead_runs) asm volatile("griddepcontrol.wait;" ::: "memory");
+  uint32_t key_cur, key_nxt;
+  bool ok_cur, ok_nxt;
+  fetch_key(keys, tile, n_tiles, tshift, n_keys, p.table.num_keys, lane, key_cur, ok_cur, bad);
+  fetch_key(keys, tile + n_warps, n_tiles, tshift, n_keys, p.table.num_keys, lane, key_nxt, ok_nxt, bad);
+  Probe<FLAT> pr;
+  probe_issue(p.table, key_cur, ok_cur, pr);
+  auto batch_index = [&](uint64_t k) {  // index of an id of the batch among the distinct ones
+    return k < p.table.num_keys ? (int32_t)(__ldcg(p.stamp + k) & kStampPending) : -1;
+  };
+  int32_t inv_idx[2];
+  if (UNIQUE) {
+#pragma unroll
+    for (int j = 0; j < 2; j++) inv_idx[j] = batch_index(inv_key[j]);
+  }
+  uint32_t word = probe_resolve(p.table, pr, key_cur, ok_cur);
+  // EARLY: the first host row of this warp's first tile is fetched before the dependency wait
+  // and held in registers, one piece per lane.
+  // CTAs of this launch become resident while the launch ahead is still waiting for ITS last
+  // host rows; their requests keep the host link's queue filled across the boundary between
+  // two launches, where it would otherwise run empty and fill up again.
+  uint32_t early_lane = 32;
+  if (EARLY && ahead_runs) {
+    const bool is_host = ok_cur && word == kEmptyWord;
+    const unsigned hmask = __ballot_sync(kFull, is_host);
+    if (hmask && p.row_bytes / VEC <= 32) {
+      early_lane = __ffs(hmask) - 1;
+      const uint32_t k = __shfl_sync(kFull, key_cur, early_lane);
+      if (lane < p.row_bytes / VEC)
+        ld_row(early, static_cast<const char*>(p.host_base) + (size_t)(k & p.host_mask) * p.row_bytes +
+                          (size_t)lane * VEC);
+    }
+    early_row = early_lane;
+  }
+  // With the extraction ahead still running the dependency wait comes as late as it can: behind the
+  // loads of this warp's first rows, and ahead of its first store (the batch ahead may have had the
+  // same output buffer).  A batch of one pass per warp then has all its loads behind it when the
+  // launch ahead ends.
   if (UNIQUE) {
     wait_for_launch_ahead();
 #pragma unroll
@@ -1155,6 +1208,7 @@ __global__ void __launch_bounds__(kBlock, DEEP ? 3 : 4)
     unsigned long long t1;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
     atomicMax(&p.counters->t_end[kGroupLocal], t1);  // one span for the whole kernel
+    if (!UNIQUE && blockIdx.x < kRunMarks) clear_running(p.order, blockIdx.x);
   }
 }
 
@@ -1853,7 +1907,7 @@ inline uint32_t host_order_shift(uint64_t host_rows) {
 cudaError_t launch_lookup_group(const void* keys, int key_bytes, uint32_t n, const TableView& table,
                                 uint32_t local_loc, uint32_t host_loc, int empty_feat,
                                 uint64_t* list_local, uint64_t* list_remote, uint64_t* list_host,
-                                Counters* counters, int keys_per_thread, uint32_t* host_hist,
+                                Counters* counters, const StreamOrder& order, int keys_per_thread, uint32_t* host_hist,
                                 uint64_t host_rows, bool pdl, cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
   const uint32_t mask = host_mask_of(empty_feat);
@@ -1863,7 +1917,7 @@ cudaError_t launch_lookup_group(const void* keys, int key_bytes, uint32_t n, con
 #define UGC_LAUNCH_LOOKUP(KEYT, KPT)                                                             \
   return launch_pdl(lookup_group_kernel<KEYT, KPT>, (int)((n + kBlock * KPT - 1) / (kBlock * KPT)), \
                     kBlock, 0, stream, pdl, static_cast<const KEYT*>(keys), n, table, local_loc,   \
-                    host_loc, mask, list_local, list_remote, list_host, counters, host_hist, shift)
+                    host_loc, mask, list_local, list_remote, list_host, counters, order, host_hist, shift)
   if (key_bytes == 8) {
     if (keys_per_thread == 1) UGC_LAUNCH_LOOKUP(long long, 1);
     if (keys_per_thread == 2) UGC_LAUNCH_LOOKUP(long long, 2);

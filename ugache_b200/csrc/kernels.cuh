@@ -20,6 +20,7 @@ namespace ugc {
 
 // All launchers enqueue on `stream` and return the launch status; none synchronises.
 
+// order: the extraction's place in its stream (order.seq is the gather's to announce).
 // keys_per_thread: 1, 2 or 4; 0 = chosen by the batch size.  host_hist: nullptr, or the scratch of
 // launch_host_order (host_order_scratch_bytes(), zero on entry), in which the host rows of the
 // batch are counted per address range of the `host_rows` rows.
@@ -27,7 +28,7 @@ namespace ugc {
 cudaError_t launch_lookup_group(const void* keys, int key_bytes, uint32_t n, const TableView& table,
                                 uint32_t local_loc, uint32_t host_loc, int empty_feat,
                                 uint64_t* list_local, uint64_t* list_remote, uint64_t* list_host,
-                                Counters* counters, int keys_per_thread, uint32_t* host_hist,
+                                Counters* counters, const StreamOrder& order, int keys_per_thread, uint32_t* host_hist,
                                 uint64_t host_rows, bool pdl, cudaStream_t stream);
 
 cudaError_t launch_gather_roles(const GatherParams& p, int grid, int block, int vec_bytes,
