@@ -220,6 +220,14 @@ def lib():
 _fast = None
 
 
+def fast_abi():
+    """What the extension module depends on besides its source: the interpreter's and torch's binary interface."""
+    import sysconfig
+
+    import torch
+    return "%s torch-%s cxx11-%d" % (sysconfig.get_config_var("SOABI"), torch.__version__, torch._C._GLIBCXX_USE_CXX11_ABI)
+
+
 def fast():
     """The extension module with the per-step calls (needs torch); raises if it has not been built."""
     global _fast
@@ -233,6 +241,9 @@ def fast():
         spec = importlib.util.spec_from_file_location("ugache_b200._fast", FAST_PATH)
         m = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(m)
+        if m.built_for != fast_abi():
+            raise ImportError("_fast.so was built for %s, this is %s: build it with `python -m ugache_b200.build`"
+                              % (m.built_for, fast_abi()))
         m.bind(check, {name: C.cast(getattr(L, name), C.c_void_p).value
                        for name in ("ugc_lookup_i64", "ugc_lookup_u32", "ugc_lookup_unique", "ugc_lookup_pool",
                                     "ugc_record")})

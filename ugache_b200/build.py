@@ -8,12 +8,14 @@ import hashlib
 import os
 import shutil
 import subprocess
+import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libugache_b200.so")
 FAST = os.path.join(HERE, "_fast.so")  # the Python face's per-step calls (links against torch)
 STAMP = os.path.join(HERE, "build", "stamp.txt")
+FAST_STAMP = os.path.join(HERE, "build", "fast_stamp.txt")
 
 CUDA_SOURCES = ["kernels.cu", "api.cu"]
 HOST_SOURCES = ["placement.cc", "compat_api.cc"]
@@ -32,47 +34,81 @@ def _nvcc():
     return nvcc
 
 
-def _fingerprint():
+def _fingerprint(names, command):
     h = hashlib.sha256()
-    for name in CUDA_SOURCES + HOST_SOURCES + [FAST_SOURCE] + HEADERS:
+    for name in names:
         path = os.path.join(CSRC, name)
         if os.path.exists(path):
             with open(path, "rb") as f:
                 h.update(name.encode())
                 h.update(f.read())
-    h.update(" ".join(NVCC_FLAGS).encode())
+    h.update(" ".join(command).encode())
     return h.hexdigest()
 
 
-def _build_fast():
-    """The extension module for the interpreter and torch that run this."""
+def _up_to_date(path, stamp, fp):
+    if not (os.path.exists(path) and os.path.exists(stamp)):
+        return False
+    with open(stamp) as f:
+        return f.read().strip() == fp
+
+
+def _write(path, text):
+    with open(path, "w") as f:
+        f.write(text)
+
+
+FAST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
+FAST_LIBS = ["-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+
+
+def build_fast(force=False):
+    """Compile the extension module if its source, the interpreter or torch changed; without torch there is
+    none (the C library does not need it)."""
+    try:
+        import torch
+
+        from ._lib import fast_abi
+        abi = fast_abi()
+    except ImportError as e:
+        print("ugache_b200: %s is not built, torch cannot be imported (%s)" % (os.path.basename(FAST), e), file=sys.stderr)
+        return
+    fp = _fingerprint([FAST_SOURCE, "../../include/ugache_b200.h"], [abi] + FAST_FLAGS + FAST_LIBS)
+    if not force and _up_to_date(FAST, FAST_STAMP, fp):
+        return
     import sysconfig
 
-    import torch
     from torch.utils import cpp_extension
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     inc = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
-    tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-           "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI, os.path.join(CSRC, FAST_SOURCE), "-o", FAST]
+    cmd = ["g++"] + FAST_FLAGS + ['-DUGC_BUILT_FOR="%s"' % abi,
+                                  "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI]
+    cmd += [os.path.join(CSRC, FAST_SOURCE), "-o", FAST]
     for i in inc:
         cmd += ["-isystem", i]
-    cmd += ["-L" + tlib, "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+    cmd += ["-L" + os.path.join(os.path.dirname(torch.__file__), "lib")] + FAST_LIBS
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("g++ failed on %s:\n%s" % (FAST_SOURCE, r.stderr))
+    _write(FAST_STAMP, fp)
 
 
 def build(force=False, verbose=False):
     """Compile the shared library and the extension module if sources changed.  Returns the library's path."""
-    fp = _fingerprint()
-    if not force and all(map(os.path.exists, (LIB, FAST, STAMP))):
-        with open(STAMP) as f:
-            if f.read().strip() == fp:
-                return LIB
+    os.makedirs(os.path.dirname(STAMP), exist_ok=True)
+    fp = _fingerprint(CUDA_SOURCES + HOST_SOURCES + HEADERS, NVCC_FLAGS)
+    if force or not _up_to_date(LIB, STAMP, fp):
+        log = _build_library()
+        _write(STAMP, fp)
+        if verbose:
+            print("\n".join(log))
+    build_fast(force)
+    return LIB
+
+
+def _build_library():
     nvcc = _nvcc()
     bdir = os.path.join(HERE, "build")
-    os.makedirs(bdir, exist_ok=True)
     objs = []
     log = []
     for src in CUDA_SOURCES + HOST_SOURCES:
@@ -91,16 +127,9 @@ def build(force=False, verbose=False):
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("link failed:\n%s" % r.stderr)
-    _build_fast()
-    with open(os.path.join(bdir, "ptxas.log"), "w") as f:
-        f.write("\n".join(log))
-    with open(STAMP, "w") as f:
-        f.write(fp)
-    if verbose:
-        print("\n".join(log))
-    return LIB
+    _write(os.path.join(bdir, "ptxas.log"), "\n".join(log))
+    return log
 
 
 if __name__ == "__main__":
-    import sys
     print(build(force="--force" in sys.argv, verbose="-v" in sys.argv))

@@ -245,4 +245,11 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_fast", nullptr, -1, kMethods, nu
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__fast() { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__fast() {
+  PyObject* m = PyModule_Create(&kModule);
+  if (m && PyModule_AddStringConstant(m, "built_for", UGC_BUILT_FOR) < 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}
