@@ -56,3 +56,31 @@ def test_host_rows_at_any_byte(built_lib, shift, zero_copy):
     assert got[shift:shift + n * row].tobytes() == table[keys.numpy()].tobytes()
     assert (got[:shift] == 7).all() and (got[shift + n * row:] == 7).all()
     cache.close()
+
+
+def test_an_error_is_reported_once(built_lib):
+    """CUDA refuses to copy to a buffer that is pinned in part; the calls after that one succeed."""
+    import ctypes as C
+    import mmap
+
+    from ugache_b200 import _lib, runtime as rt
+    N, dim, page = 5000, 32, 4096
+    table = np.arange(N * dim, dtype=np.float32).reshape(N, dim)
+    host = torch.from_numpy(table).pin_memory()
+    keys = torch.arange(200).pin_memory()
+    area = mmap.mmap(-1, 8 * page)
+    base = C.addressof(C.c_char.from_buffer(area))
+    stream = torch.cuda.current_stream().cuda_stream
+    cudart = torch.cuda.cudart()
+    assert int(cudart.cudaHostRegister(base, page, 0)) == 0
+    for _ in range(2):
+        cache = rt.Cache(1, N, dim * 4, 0.5, max_batch=1024)
+        cache.set_placement(rt.solve_placement("rep", 1, np.arange(N, dtype=np.uint32), None, 50.0))
+        cache.build(0, 0, host.data_ptr())
+        cache.tune(0, host_zero_copy=0)
+        with pytest.raises(_lib.UgcError, match="cudaMemcpyAsync"):
+            cache.lookup_host_ptr(0, keys.data_ptr(), 8, 200, base, stream)
+        cache.record(0, keys.cuda())
+        assert cache.hotness_read(0, stream=stream).sum() == 200
+        cache.close()
+    cudart.cudaHostUnregister(base)

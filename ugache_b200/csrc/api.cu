@@ -49,9 +49,11 @@ int fail(int code, const char* fmt, ...) {
 #define UGC_CUDA(expr)                                                                        \
   do {                                                                                        \
     cudaError_t e__ = (expr);                                                                 \
-    if (e__ != cudaSuccess)                                                                   \
+    if (e__ != cudaSuccess) {                                                                 \
+      cudaGetLastError(); /* reported here: the next launch must not find it again */         \
       return fail(UGC_ERR_CUDA, "%s failed: %s (%s:%d)", #expr, cudaGetErrorString(e__),     \
                   __FILE__, __LINE__);                                                        \
+    }                                                                                         \
   } while (0)
 
 #define UGC_TRY(expr)              \
