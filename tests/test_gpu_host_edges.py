@@ -84,3 +84,48 @@ def test_an_error_is_reported_once(built_lib):
         assert cache.hotness_read(0, stream=stream).sum() == 200
         cache.close()
     cudart.cudaHostUnregister(base)
+
+# Buffers pinned at both ends with a pageable hole between, and at the start only, are not used in place
+# (CUDA refuses to copy them); ones pinned in two pieces are
+@pytest.mark.parametrize("pinned,whole", [(((0, 1), (6, 8)), False), (((0, 3),), False), (((0, 4), (4, 8)), True)])
+@pytest.mark.parametrize("zero_copy", [1, 3])
+def test_host_buffers_pinned_in_part(built_lib, pinned, whole, zero_copy):
+    import ctypes as C
+    import mmap
+
+    from ugache_b200 import _lib, runtime as rt, workload as wl
+    N, dim, page = 5000, 32, 4096
+    row, n = dim * 4, 8 * page // (dim * 4)
+    table = wl.table(4, N, dim)
+    ids, freqs = wl.analytic_hotness(N, 1.1)
+    cache = rt.Cache(1, N, row, 0.5, max_batch=8192)
+    cache.set_placement(rt.solve_placement("intuitive", 1, ids, freqs, 50.0))
+    host = torch.from_numpy(table).pin_memory()
+    cache.build(0, 0, host.data_ptr())
+    cache.tune(0, host_zero_copy=zero_copy)
+    areas = [mmap.mmap(-1, 8 * page) for _ in range(2)]
+    base = [C.addressof(C.c_char.from_buffer(m)) for m in areas]
+    cudart = torch.cuda.cudart()
+    for b in base:
+        for lo, hi in pinned:
+            assert int(cudart.cudaHostRegister(b + lo * page, (hi - lo) * page, 0)) == 0
+    stream = torch.cuda.current_stream().cuda_stream
+    area, key_area = (np.frombuffer(m, dtype=np.uint8) for m in areas)
+    k = wl.zipf_keys(3, 8 * page // 8, N, 1.1)
+    key_area.view(np.int64)[:] = k
+    own_keys = torch.from_numpy(k).pin_memory()
+    own_out = torch.zeros((len(k), dim)).pin_memory()
+    calls = [(own_keys.data_ptr(), n, base[0], area), (base[1], len(k), own_out.data_ptr(), own_out.numpy())]
+    for keys_ptr, count, out_ptr, out in calls:      # as many rows, or keys, as the area holds
+        if whole:
+            cache.lookup_host_ptr(0, keys_ptr, 8, count, out_ptr, stream)
+            assert out.tobytes() == table[k[:count]].tobytes()
+        else:
+            with pytest.raises(_lib.UgcError):
+                cache.lookup_host_ptr(0, keys_ptr, 8, count, out_ptr, stream)
+    cache.lookup_host_ptr(0, own_keys.data_ptr(), 8, len(k), own_out.data_ptr(), stream)
+    assert own_out.numpy().tobytes() == table[k].tobytes()
+    for b in base:
+        for lo, hi in pinned:
+            cudart.cudaHostUnregister(b + lo * page)
+    cache.close()

@@ -1005,15 +1005,31 @@ GatherParams gather_params(ugc_ctx* c, Replica* r, void* out, uint32_t n) {
   return p;
 }
 
-// Device-side address of pinned host memory that the GPU has mapped, else nullptr.
-void* mapped_device_pointer(const void* host) {
-  cudaPointerAttributes attr;
-  if (cudaPointerGetAttributes(&attr, host) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
+// Device-side address of `bytes` of pinned host memory that the GPU has mapped, every one of them, else
+// nullptr: a caller may have pinned a part, or both ends.
+void* mapped_device_pointer(const void* host, size_t bytes) {
+  static CUresult (*const attribute)(void*, CUpointer_attribute, CUdeviceptr) = [] {
+    CUresult (*fn)(void*, CUpointer_attribute, CUdeviceptr) = nullptr;
+    return resolve("cuPointerGetAttribute", &fn) ? fn : nullptr;
+  }();
+  char* dev = nullptr;
+  for (size_t at = 0; at < bytes;) {  // one registration after the other; most buffers lie in one
+    cudaPointerAttributes attr;
+    if (!attribute || cudaPointerGetAttributes(&attr, static_cast<const char*>(host) + at) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    if (attr.type != cudaMemoryTypeHost || !attr.devicePointer) return nullptr;
+    if (at == 0) dev = static_cast<char*>(attr.devicePointer);
+    const CUdeviceptr p = reinterpret_cast<CUdeviceptr>(attr.devicePointer);
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    if (attr.devicePointer != dev + at || attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, p) != CUDA_SUCCESS ||
+        attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, p) != CUDA_SUCCESS || p < start || p - start >= size)
+      return nullptr;
+    at += size - (p - start);
   }
-  if (attr.type != cudaMemoryTypeHost || !attr.devicePointer) return nullptr;
-  return attr.devicePointer;
+  return dev;
 }
 
 // The last few streams lookups of this replica were enqueued on (most callers use one).
@@ -2050,14 +2066,11 @@ int ugc_lookup_host(ugc_ctx* c, int replica_id, const void* keys, int key_bytes,
   UGC_CUDA(cudaSetDevice(r->device));
   // Pinned buffers that the GPU has mapped are used in place: the kernel reads the keys and
   // writes the rows across PCIe itself.
-  const void* keys_dev = (r->host_zero_copy & 1) ? mapped_device_pointer(keys) : nullptr;
+  const void* keys_dev = (r->host_zero_copy & 1) ? mapped_device_pointer(keys, n * (size_t)key_bytes) : nullptr;
   const size_t rb = c->cfg.row_bytes;
   void* out_dev = nullptr;
-  if (rows_in_place(r->host_zero_copy, n * rb, reinterpret_cast<uintptr_t>(out) | rb)) {
-    out_dev = mapped_device_pointer(out);
-    const char* last = static_cast<const char*>(out) + (n * rb - 1);  // the caller may have pinned a part
-    if (out_dev && mapped_device_pointer(last) != static_cast<char*>(out_dev) + (n * rb - 1)) out_dev = nullptr;
-  }
+  if (rows_in_place(r->host_zero_copy, n * rb, reinterpret_cast<uintptr_t>(out) | rb))
+    out_dev = mapped_device_pointer(out, n * rb);
   if (!keys_dev) {
     UGC_TRY(ensure(c, r->stage_keys, n * (size_t)key_bytes));
     UGC_CUDA(cudaMemcpyAsync(r->stage_keys.ptr, keys, n * (size_t)key_bytes, cudaMemcpyHostToDevice, s));
