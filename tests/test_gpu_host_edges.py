@@ -129,3 +129,22 @@ def test_host_buffers_pinned_in_part(built_lib, pinned, whole, zero_copy):
         for lo, hi in pinned:
             cudart.cudaHostUnregister(b + lo * page)
     cache.close()
+
+
+# Keys at an address that is not a multiple of their size are staged
+@pytest.mark.parametrize("key_bytes,shift", [(8, 1), (8, 4), (4, 1), (4, 2)])
+def test_host_keys_at_any_byte(built_lib, key_bytes, shift):
+    from ugache_b200 import runtime as rt
+    N, dim, n = 5000, 32, 300
+    table = np.arange(N * dim, dtype=np.float32).reshape(N, dim)
+    cache = rt.Cache(1, N, dim * 4, 0.5, max_batch=1024)
+    cache.set_placement(rt.solve_placement("rep", 1, np.arange(N, dtype=np.uint32), None, 50.0))
+    host = torch.from_numpy(table).pin_memory()
+    cache.build(0, 0, host.data_ptr())
+    keys = np.random.default_rng(1).integers(0, N, n).astype(np.int64 if key_bytes == 8 else np.int32)
+    raw = torch.zeros(shift + keys.nbytes, dtype=torch.uint8).pin_memory()
+    raw.numpy()[shift:] = keys.view(np.uint8)
+    out = torch.zeros((n, dim)).pin_memory()
+    cache.lookup_host_ptr(0, raw.data_ptr() + shift, key_bytes, n, out.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert np.array_equal(out.numpy(), table[keys])
+    cache.close()

@@ -2066,7 +2066,9 @@ int ugc_lookup_host(ugc_ctx* c, int replica_id, const void* keys, int key_bytes,
   UGC_CUDA(cudaSetDevice(r->device));
   // Pinned buffers that the GPU has mapped are used in place: the kernel reads the keys and
   // writes the rows across PCIe itself.
-  const void* keys_dev = (r->host_zero_copy & 1) ? mapped_device_pointer(keys, n * (size_t)key_bytes) : nullptr;
+  const bool keys_aligned = reinterpret_cast<uintptr_t>(keys) % (uintptr_t)key_bytes == 0;  // else staged
+  const void* keys_dev =
+      (r->host_zero_copy & 1) && keys_aligned ? mapped_device_pointer(keys, n * (size_t)key_bytes) : nullptr;
   const size_t rb = c->cfg.row_bytes;
   void* out_dev = nullptr;
   if (rows_in_place(r->host_zero_copy, n * rb, reinterpret_cast<uintptr_t>(out) | rb))
