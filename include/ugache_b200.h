@@ -430,7 +430,7 @@ typedef struct {
   int32_t programmatic_launch;    /* programmatic stream serialization: bit 0 for the lookup
                                      kernel (its key loads and probes overlap the tail of
                                      the previous gather) and for deduplicated and pooled
-                                     lookups, bit 1 for the gather kernel (it is
+                                     lookups and ugc_record, bit 1 for the gather kernel (it is
                                      scheduled while the lookup kernel drains)              */
   int32_t extract_mode;           /* ugc_extract_mode                                       */
   int32_t direct_ctas_per_sm;     /* CTAs of the direct extraction kernel per SM, 1..16     */

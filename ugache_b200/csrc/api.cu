@@ -2313,7 +2313,8 @@ int ugc_record(ugc_ctx* c, int replica_id, const void* keys, int key_bytes, size
     if (!r->hot_counts) return fail(UGC_ERR_NOMEM, "hotness counters (%zu bytes) could not be allocated", bytes);
     UGC_CUDA(cudaMemsetAsync(r->hot_counts, 0, bytes, s));
   }
-  UGC_CUDA(launch_record(keys, key_bytes, (uint32_t)n, r->hot_counts, c->cfg.num_total_item, s));
+  UGC_CUDA(launch_record(keys, key_bytes, (uint32_t)n, r->hot_counts, c->cfg.num_total_item,
+                         (r->pdl & 1) != 0, s));
   return UGC_OK;
 }
 

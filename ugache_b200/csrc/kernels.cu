@@ -2159,13 +2159,13 @@ cudaError_t launch_classify_scatter(const ClassifyParams& p, const void* scratch
 }
 
 cudaError_t launch_record(const void* keys, int key_bytes, uint32_t n, uint32_t* counts,
-                          uint64_t num_keys, cudaStream_t stream) {
+                          uint64_t num_keys, bool pdl, cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
   const int grid = (int)(((uint64_t)n + kBlock * kRecordKpt - 1) / (kBlock * kRecordKpt));
   if (key_bytes == 8)
-    return launch_pdl(record_kernel<long long>, grid, kBlock, 0, stream, true,
+    return launch_pdl(record_kernel<long long>, grid, kBlock, 0, stream, pdl,
                       static_cast<const long long*>(keys), n, counts, num_keys);
-  return launch_pdl(record_kernel<uint32_t>, grid, kBlock, 0, stream, true,
+  return launch_pdl(record_kernel<uint32_t>, grid, kBlock, 0, stream, pdl,
                     static_cast<const uint32_t*>(keys), n, counts, num_keys);
 }
 
