@@ -515,8 +515,10 @@ struct PinnedBlock {
 };
 
 // Pinned staging between pageable host arrays and the GPU: one block of kStageParts parts for the
-// whole process, taken by one build / refresh / hotness step at a time, which leaves no copy in
-// flight behind.  Made on first use (2-3 ms: per cache it would be a third of a small build) and
+// whole process, taken by one build / refresh / hotness step at a time (StageUse).  Its copies run on a
+// stream of the replica's own once the caller's stream is idle, so that whoever holds the block waits
+// for nothing but those copies, and none is in flight when the block is given back, failures included.
+// Made on first use (2-3 ms: per cache it would be a third of a small build) and
 // given back with the last context.
 constexpr uint64_t kStageKeys = 1u << 19;
 constexpr int kStageParts = 4;
@@ -602,6 +604,7 @@ struct Replica {
   uint8_t* src_next = nullptr;             // same for the placement a refresh is moving to
   PinnedBlock* pinned = nullptr;
   cudaEvent_t stage_ev[kStageParts] = {};
+  cudaStream_t stage_stream = nullptr;     // copies through the staging block
   DevBuf class_scratch;
   DevBuf lists;                            // all lists back to back
   uint64_t list_count[kMaxClassLists] = {0};
@@ -891,6 +894,27 @@ int make_stage() {
   return UGC_OK;
 }
 
+class StageUse {
+ public:
+  // Waits for the caller's stream (before the block is taken), then for the block.
+  int take(Replica* r, cudaStream_t caller) {
+    UGC_CUDA(cudaEventRecord(r->stage_ev[0], caller));  // (on the default stream: behind all blocking ones)
+    UGC_CUDA(cudaEventSynchronize(r->stage_ev[0]));
+    if (!r->stage_stream) UGC_CUDA(cudaStreamCreateWithFlags(&r->stage_stream, cudaStreamNonBlocking));
+    lock_ = std::unique_lock<std::mutex>(g_stage_mu);
+    stream_ = r->stage_stream;
+    return make_stage();
+  }
+  ~StageUse() {
+    if (stream_) cudaStreamSynchronize(stream_);
+  }
+  cudaStream_t stream() const { return stream_; }
+
+ private:
+  std::unique_lock<std::mutex> lock_;  // released after the destructor's body
+  cudaStream_t stream_ = nullptr;
+};
+
 // This reader's source of every key as one byte per key on the device: block_access_from[me] at
 // nid_to_block[key], looked up by the host threads on the way into the pinned staging buffer.
 // One byte instead of four crosses PCIe, at the pinned rate, and the classification reads a
@@ -906,8 +930,12 @@ int upload_sources(ugc_ctx* c, Replica* r, const Placement& p, uint8_t** dst, cu
   const uint8_t* acc = &p.block_access_from[(size_t)r->id * p.num_block];
   const uint32_t* n2b = p.nid_to_block.data();
   const int threads = std::max(1, std::min(16, omp_get_num_procs()));
-  std::lock_guard<std::mutex> lock(g_stage_mu);
-  if (!r->built && !g_stage && N <= (8u << 20)) {
+  bool have_stage;
+  {
+    std::lock_guard<std::mutex> lock(g_stage_mu);
+    have_stage = g_stage != nullptr;
+  }
+  if (!r->built && !have_stage && N <= (8u << 20)) {
     std::unique_ptr<uint8_t[]> bytes(new (std::nothrow) uint8_t[N]);
     if (!bytes) return fail(UGC_ERR_NOMEM, "out of host memory");
 #pragma omp parallel for schedule(static) num_threads(N > 65536 ? threads : 1)
@@ -916,7 +944,8 @@ int upload_sources(ugc_ctx* c, Replica* r, const Placement& p, uint8_t** dst, cu
     UGC_CUDA(cudaStreamSynchronize(s));
     return UGC_OK;
   }
-  UGC_TRY(make_stage());
+  StageUse use;
+  UGC_TRY(use.take(r, s));
   int buf = 0;
   for (uint64_t off = 0; off < N; off += kStageKeys, buf = (buf + 1) % kStageParts) {
     const int64_t m = (int64_t)std::min<uint64_t>(kStageKeys, N - off);
@@ -925,10 +954,10 @@ int upload_sources(ugc_ctx* c, Replica* r, const Placement& p, uint8_t** dst, cu
     const uint32_t* from = n2b + off;
 #pragma omp parallel for schedule(static) num_threads(m > 65536 ? threads : 1)
     for (int64_t i = 0; i < m; i++) stage[i] = acc[from[i]];
-    UGC_CUDA(cudaMemcpyAsync(*dst + off, stage, (size_t)m, cudaMemcpyHostToDevice, s));
-    UGC_CUDA(cudaEventRecord(r->stage_ev[buf], s));
+    UGC_CUDA(cudaMemcpyAsync(*dst + off, stage, (size_t)m, cudaMemcpyHostToDevice, use.stream()));
+    UGC_CUDA(cudaEventRecord(r->stage_ev[buf], use.stream()));
   }
-  for (auto& e : r->stage_ev) UGC_CUDA(cudaEventSynchronize(e));
+  UGC_CUDA(cudaStreamSynchronize(use.stream()));
   return UGC_OK;
 }
 
@@ -962,6 +991,7 @@ void release_replica(ugc_ctx* c, Replica* r) {
   if (r->pinned) cudaFreeHost(r->pinned);
   for (cudaEvent_t e : r->stage_ev)
     if (e) cudaEventDestroy(e);
+  if (r->stage_stream) cudaStreamDestroy(r->stage_stream);
   *r = Replica{};
 }
 
@@ -2332,8 +2362,8 @@ int ugc_hotness_read(ugc_ctx* c, int replica_id, uint32_t* counts_out, int reset
   // The caller's array is pageable: the counters come through the parts of the pinned staging
   // block, up to three crossing PCIe while the host threads copy the oldest out (8 MB: 450-680 us
   // through the driver's own staging, which copies with one thread).
-  std::lock_guard<std::mutex> lock(g_stage_mu);
-  UGC_TRY(make_stage());
+  StageUse use;
+  UGC_TRY(use.take(r, s));
   const int threads = std::max(1, std::min(16, omp_get_num_procs()));
   const size_t pieces = (bytes + kStageKeys - 1) / kStageKeys;
   auto length = [&](size_t i) { return std::min<size_t>(kStageKeys, bytes - i * kStageKeys); };
@@ -2342,8 +2372,8 @@ int ugc_hotness_read(ugc_ctx* c, int replica_id, uint32_t* counts_out, int reset
     for (; sent < pieces && sent < i + kStageParts; sent++) {
       const int buf = (int)(sent % kStageParts);
       UGC_CUDA(cudaMemcpyAsync(g_stage + buf * kStageKeys, reinterpret_cast<const char*>(r->hot_counts) + sent * kStageKeys,
-                               length(sent), cudaMemcpyDeviceToHost, s));
-      UGC_CUDA(cudaEventRecord(r->stage_ev[buf], s));
+                               length(sent), cudaMemcpyDeviceToHost, use.stream()));
+      UGC_CUDA(cudaEventRecord(r->stage_ev[buf], use.stream()));
     }
     const int64_t len = (int64_t)length(i);
     const uint8_t* from = g_stage + (i % kStageParts) * kStageKeys;
