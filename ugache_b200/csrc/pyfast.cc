@@ -87,10 +87,20 @@ bool arg_count(Py_ssize_t n, Py_ssize_t want) {
   return false;
 }
 
+// C++ exceptions become the Python ones torch raises for them (by its translation alone: the buffer for
+// warnings that torch's own macros set up besides would be made on every call)
+#define UGC_PY_TRY try {
+#define UGC_PY_END                                                  \
+  }                                                                 \
+  catch (...) {                                                     \
+    torch::translate_exception_to_python(std::current_exception()); \
+    return nullptr;                                                 \
+  }
+
 // lookup(ctx, replica, row_bytes, keys, out | None, stream | None) -> out
 PyObject* fast_lookup(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   if (!arg_count(n_args, 6)) return nullptr;
-  HANDLE_TH_ERRORS  // C++ exceptions become the Python ones torch raises for them
+  UGC_PY_TRY
   ugc_ctx* ctx = static_cast<ugc_ctx*>(PyLong_AsVoidPtr(a[0]));
   const int replica = (int)PyLong_AsLong(a[1]);
   const int64_t row_bytes = PyLong_AsLongLong(a[2]);
@@ -117,13 +127,13 @@ PyObject* fast_lookup(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   if (rc != UGC_OK) return raise_status(rc);
   if (!made.defined()) return Py_NewRef(a[4]);
   return THPVariable_Wrap(std::move(made));
-  END_HANDLE_TH_ERRORS
+  UGC_PY_END
 }
 
 // lookup_unique(ctx, replica, row_bytes, keys, stream | None) -> (rows, unique_keys, inverse, n_unique)
 PyObject* fast_lookup_unique(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   if (!arg_count(n_args, 5)) return nullptr;
-  HANDLE_TH_ERRORS
+  UGC_PY_TRY
   ugc_ctx* ctx = static_cast<ugc_ctx*>(PyLong_AsVoidPtr(a[0]));
   const int replica = (int)PyLong_AsLong(a[1]);
   const int64_t row_bytes = PyLong_AsLongLong(a[2]);
@@ -154,14 +164,14 @@ PyObject* fast_lookup_unique(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   PyTuple_SET_ITEM(t, 2, THPVariable_Wrap(std::move(inverse)));
   PyTuple_SET_ITEM(t, 3, THPVariable_Wrap(std::move(n_unique)));
   return t;
-  END_HANDLE_TH_ERRORS
+  UGC_PY_END
 }
 
 // lookup_pool(ctx, replica, keys, offsets | None, n_bags, bag_size, elem_type, mode, dim, out | None,
 //             stream | None) -> out
 PyObject* fast_lookup_pool(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   if (!arg_count(n_args, 11)) return nullptr;
-  HANDLE_TH_ERRORS
+  UGC_PY_TRY
   ugc_ctx* ctx = static_cast<ugc_ctx*>(PyLong_AsVoidPtr(a[0]));
   const int replica = (int)PyLong_AsLong(a[1]);
   const int64_t n_bags = PyLong_AsLongLong(a[4]), bag_size = PyLong_AsLongLong(a[5]);
@@ -190,13 +200,13 @@ PyObject* fast_lookup_pool(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   if (rc != UGC_OK) return raise_status(rc);
   if (!made.defined()) return Py_NewRef(a[9]);
   return THPVariable_Wrap(std::move(made));
-  END_HANDLE_TH_ERRORS
+  UGC_PY_END
 }
 
 // record(ctx, replica, keys, stream | None)
 PyObject* fast_record(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   if (!arg_count(n_args, 4)) return nullptr;
-  HANDLE_TH_ERRORS
+  UGC_PY_TRY
   ugc_ctx* ctx = static_cast<ugc_ctx*>(PyLong_AsVoidPtr(a[0]));
   const int replica = (int)PyLong_AsLong(a[1]);
   if (PyErr_Occurred()) return nullptr;
@@ -212,7 +222,7 @@ PyObject* fast_record(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   Py_END_ALLOW_THREADS
   if (rc != UGC_OK) return raise_status(rc);
   Py_RETURN_NONE;
-  END_HANDLE_TH_ERRORS
+  UGC_PY_END
 }
 
 // bind(check, {entry point name: address})
