@@ -103,8 +103,9 @@ typedef struct {
                                  host link full by ugc_link_desc                         */
   int32_t remote_ctas;        /* most CTAs the peer-row group may take; 0 = what keeps the
                                  NVLink port full by ugc_link_desc                       */
-  int32_t gather_vec_bytes;   /* 16 or 32 bytes per lane per load in the gather (host rows
-                                 always use 16); 0 = 32 with 8 GPUs, else 16            */
+  int32_t gather_vec_bytes;   /* 16 or 32 bytes per lane per load in the extraction (the
+                                 gather's host rows always use 16); 0 = 32 with 8 GPUs,
+                                 else 16                                                */
   ugc_alloc_fn alloc;
   ugc_free_fn free;
   void* alloc_user;
@@ -420,7 +421,8 @@ typedef struct {
   uint32_t struct_size;
   int32_t gather_ctas_per_sm;     /* CTAs of the gather kernel per SM                       */
   int32_t gather_block_threads;   /* 256, 512 or 1024                                       */
-  int32_t gather_vec_bytes;       /* 16 or 32 bytes per lane per load of the gather         */
+  int32_t gather_vec_bytes;       /* 16 or 32 bytes per lane per load of the gather and of the
+                                     direct kernel                                           */
   int32_t host_ctas;              /* most CTAs the host-row group may take (left at its default: fewer
                                      for a host list in address order and rows below 1 KB)   */
   int32_t remote_ctas;            /* most CTAs the peer-row group may take                       */

@@ -1,0 +1,41 @@
+"""The rules that pick a load width, a path and a number of CTAs: whatever they pick, rows are equal or wrong."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def build(table, share, max_batch, **kw):
+    from ugache_b200 import runtime as rt
+    N, row = len(table), table.nbytes // len(table)
+    cache = rt.Cache(1, N, row, share, max_batch=max_batch, **kw)
+    cache.set_placement(rt.solve_placement("rep", 1, np.arange(N, dtype=np.uint32), None, share * 100.0))
+    host = torch.from_numpy(table.view(np.uint8).reshape(N, row)).pin_memory()
+    cache.build(0, 0, host.data_ptr())
+    cache._keep.append(host)
+    return cache
+
+
+@pytest.mark.parametrize("kind", [1, 2])           # direct-index and probing table
+def test_load_width_is_a_choice_again(built_lib, kind):
+    from ugache_b200 import _lib
+    table = np.random.default_rng(1).integers(0, 1 << 30, (20_000, 32)).astype(np.int32)
+    cache = build(table, 0.2, 8192, table_kind=kind)
+    assert cache.get_tuning(0)["gather_vec_bytes"] == 16
+    keys = torch.randint(0, 20_000, (8000,), device="cuda")
+    want = table[keys.cpu().numpy()]
+    for vec in (16, 32):
+        for mode in (_lib.EXTRACT_DIRECT, _lib.EXTRACT_GROUPED):
+            for early in (1, 2):
+                cache.tune(0, gather_vec_bytes=vec, extract_mode=mode, direct_early_host=early)
+                assert cache.get_tuning(0)["gather_vec_bytes"] == vec
+                for _ in range(2):
+                    got = cache.lookup(0, keys).view(torch.int32).cpu().numpy()
+                    assert np.array_equal(got, want), (vec, mode)
+    with pytest.raises(_lib.UgcError):
+        cache.tune(0, gather_vec_bytes=8)
+    cache.close()
+    wide = build(table, 0.2, 8192, gather_vec_bytes=32)
+    assert wide.get_tuning(0)["gather_vec_bytes"] == 32
+    wide.close()

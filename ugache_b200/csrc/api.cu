@@ -1272,7 +1272,7 @@ int do_lookup(ugc_ctx* c, Replica* r, const void* keys, int key_bytes, size_t n,
       const volatile Feedback* f = r->feedback;
       early = f->seq != 0 && f->count[kGroupHost] >= 1024u;
     }
-    UGC_CUDA(launch_extract_direct(keys, key_bytes, d, r->direct_grid, r->direct_block, r->direct_deep != 0,
+    UGC_CUDA(launch_extract_direct(keys, key_bytes, d, r->direct_grid, r->direct_block, r->vec_bytes, r->direct_deep != 0,
                                    early && d.host_base != nullptr, (r->pdl & 1) != 0, s));
     if (prof) {
       UGC_CUDA(cudaEventRecord(r->prof_events[r->prof_used + 2], s));
@@ -1643,11 +1643,14 @@ int ugc_build(ugc_ctx* c, int replica_id, int device_id, const void* host_table,
     r->t_byte[kGroupRemote] = ld.bw_remote_gbs > 0 ? (float)(1.0 / ld.bw_remote_gbs) : 0.0f;
     r->t_byte[kGroupHost] = (float)(1.0 / ld.bw_host_gbs);
   }
-  // Loads of the gather: 32 bytes win when almost every row comes from HBM (8 GPUs, 458 host rows
-  // per batch: 36.5 us per step against 45); with more host rows per batch 16-byte loads were faster
-  // (1 GPU: 113 vs 133 us, 2 GPUs: 84 vs 110 us, 4 GPUs: 54 vs 61 us).  The direct kernel takes the
-  // widest the addresses allow (90.0 against 93.5 us with 7,277 host rows per batch, 2.4 against 2.6
-  // for 208 keys, equal without host rows).
+  // Loads of both extractions.  32 bytes win when almost every row comes from HBM and it is one of
+  // eight (8 GPUs, 458 host rows per batch: 36.5 us per step against 45); else 16-byte loads are faster
+  // under a skewed batch (1 GPU: 113 vs 133 us, 2 GPUs: 84 vs 110, 4 GPUs: 54 vs 61 grouped; direct,
+  // 212,992 keys with 3,217 host rows of a 51 GB table, whose probing-table variant spills at 32: 84.1 vs
+  // 89.6; 1.47 M keys of 256-byte rows 113 vs 117; 212,992 with 592 host rows 25.7 vs 25.5 over three
+  // caches in turn and 22.5 vs 25.2 over one; 63,360 keys of 128-byte rows 6.3 vs 6.2; equal for 208 and
+  // 13,312).  Keys spread evenly over the cached rows would do better with 32 (1 GB table, 512-byte rows:
+  // 44.5 vs 39.8 with 1,024 host rows; 32 GB: within 3 %), but batches are skewed.
   r->vec_bytes = c->cfg.gather_vec_bytes ? (c->cfg.gather_vec_bytes == 32 ? 32 : 16) : (G >= 8 ? 32 : 16);
 
   // a build that fails gives everything back once the stream is done with it: a caller's allocator

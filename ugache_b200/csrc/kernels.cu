@@ -1940,12 +1940,13 @@ int usable_vec_bytes(uint32_t row_bytes, int want, const void* out, const void* 
 }
 
 cudaError_t launch_extract_direct(const void* keys, int key_bytes, const DirectParams& p_in, int grid,
-                                  int block, bool deep, bool early_host, bool pdl, cudaStream_t stream) {
+                                  int block, int vec_bytes, bool deep, bool early_host, bool pdl,
+                                  cudaStream_t stream) {
   if (block != 128 && block != 256) block = kBlock;
   const int warps_per_block = block / 32;
   if (p_in.n_keys == 0) return cudaSuccess;
   DirectParams p = p_in;
-  const int vec = usable_vec_bytes(p.row_bytes, 32, p.out, p.src_base, kMaxLocation);
+  const int vec = usable_vec_bytes(p.row_bytes, vec_bytes, p.out, p.src_base, kMaxLocation);
   const int lpr = lanes_per_row(p.row_bytes, vec);
   p.lpr_shift = 0;
   while ((1 << p.lpr_shift) < lpr) p.lpr_shift++;
