@@ -39,3 +39,18 @@ def test_load_width_is_a_choice_again(built_lib, kind):
     wide = build(table, 0.2, 8192, gather_vec_bytes=32)
     assert wide.get_tuning(0)["gather_vec_bytes"] == 32
     wide.close()
+
+
+# rows of more than 128 bytes over at most 1.5 GB go grouped from 4096 host rows on, others from 8192
+@pytest.mark.parametrize("row,nbytes,line", [(512, 1 << 26, 4096), (128, 1 << 26, 8192), (132, 1 << 26, 4096),
+                                             (512, 3 << 29, 4096), (512, (3 << 29) + 512, 8192)])
+def test_line_between_direct_and_grouped(built_lib, row, nbytes, line):
+    from ugache_b200 import runtime as rt
+    N = nbytes // row
+    host, _ = rt.host_alloc(N * row)
+    cache = rt.Cache(1, N, row, 0.001, max_batch=1024)
+    cache.set_placement(rt.solve_placement("rep", 1, np.arange(N, dtype=np.uint32), None, 0.1))
+    cache.build(0, 0, host)
+    assert cache.get_tuning(0)["direct_max_host_rows"] == line
+    cache.close()
+    rt.host_free(host)

@@ -42,3 +42,23 @@ def test_pool_edges(built_lib, dim, dtype, piece):
             assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), (name, mode)
     assert cache.stats(0)["err_key_range"] > 0
     cache.close()
+
+
+@pytest.mark.parametrize("piece", [4, 16])
+def test_pool_over_the_probing_table(built_lib, piece):
+    from ugache_b200 import _lib, runtime as rt, workload as wl
+    N, dim, n = 50_000, 64, 6000
+    table = wl.table(3, N, dim)
+    cache = rt.Cache(1, N, dim * 4, 0.05, max_batch=n, table_kind=_lib.TABLE_HASHED)
+    cache.set_placement(rt.solve_placement("rep", 1, np.arange(N, dtype=np.uint32), None, 5.0))
+    host = torch.from_numpy(table).pin_memory()
+    cache.build(0, 0, host.data_ptr())
+    cache.tune(0, pool_vec_bytes=piece)
+    keys = wl.zipf_keys(9, n, N, 1.1)
+    k = torch.from_numpy(keys).cuda()
+    off = np.array([0, 0, 5, 700, 701, n], dtype=np.int64)
+    for mode in ("sum", "mean"):
+        got = cache.lookup_pool(0, k, offsets=torch.from_numpy(off).cuda(), mode=mode).cpu().numpy()
+        want = orc.pool(table, keys, offsets=off, mean=mode == "mean")
+        assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+    cache.close()

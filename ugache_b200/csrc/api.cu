@@ -592,7 +592,7 @@ struct Replica {
   cudaStream_t recent_streams[4] = {nullptr, nullptr, nullptr, nullptr};  // streams lookups ran on
   bool recent_valid[4] = {false, false, false, false};
   int direct_block = 256;
-  int direct_max_host_rows = 4096;
+  int direct_max_host_rows = 8192;
   int direct_tile_shift = 0;               // 0: chosen per launch
   int direct_deep = 0;
   int direct_early_host = 0;               // 0 auto, 1 always, 2 never
@@ -1663,6 +1663,16 @@ int ugc_build(ugc_ctx* c, int replica_id, int device_id, const void* host_table,
     return rc;
   };
   int rc;
+  // Auto mode's line between direct and grouped.  Host rows scattered over a table that the host link's
+  // address translation covers are bound by bytes, and the grouped path moves more of them at a time;
+  // over a larger table they are bound by the rows in flight, and the direct kernel, whose every warp
+  // asks for the ones it meets, has more.  212,992 keys, 6,144 of them on the host, direct / grouped us:
+  // 512-byte rows over 1 GB 86 / 73, 2 GB 92 / 81, 4 GB 92 / 152, 8 GB 105 / 172, 32 GB 121 / 190;
+  // 200-byte rows 70 / 59, 73 / 63, 84 / 129, 105 / 182, 96 / 261.  Rows of 128 bytes are better off
+  // direct over 1 GB too (27 / 31).
+  const uint64_t table_rows = c->cfg.empty_feat > 0 ? ((uint64_t)1 << c->cfg.empty_feat) : N;
+  if (c->cfg.row_bytes > 128 && table_rows * c->cfg.row_bytes <= 3ull << 29) r->direct_max_host_rows = 4096;
+
   // 1. which source serves each key: ascending key lists per GPU source, made on the GPU
   if ((rc = make_pinned(r)) != UGC_OK) return bail(rc);
   if ((rc = upload_sources(c, r, c->cur, &r->src_dev, s)) != UGC_OK) return bail(rc);
