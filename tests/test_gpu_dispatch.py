@@ -54,3 +54,23 @@ def test_line_between_direct_and_grouped(built_lib, row, nbytes, line):
     assert cache.get_tuning(0)["direct_max_host_rows"] == line
     cache.close()
     rt.host_free(host)
+
+
+# host lists in address order: rows that move in 4-byte pieces, in odd numbers of 16-byte ones, in whole
+# ones; with and without rows in the slice
+@pytest.mark.parametrize("dim", [1, 25, 50, 100, 128, 256])
+@pytest.mark.parametrize("share", [0.0, 0.3])
+def test_ordered_host_lists(built_lib, dim, share):
+    from ugache_b200 import _lib
+    N, n = 30_000, 20_000
+    table = np.random.default_rng(dim).integers(0, 1 << 30, (N, dim)).astype(np.int32)
+    cache = build(table, share, n)
+    cache.tune(0, extract_mode=_lib.EXTRACT_GROUPED, host_order_min_rows=1)
+    batches = [torch.randint(0, N, (k,), device="cuda") for k in (n, 1, n - 7, 33)]
+    cache.lookup(0, batches[0])
+    torch.cuda.synchronize()                   # from here on the last lookup's host rows are known
+    got = [cache.lookup(0, k) for k in batches * 3]
+    for k, g in zip(batches * 3, got):
+        assert np.array_equal(g.view(torch.int32).cpu().numpy(), table[k.cpu().numpy()])
+    assert cache.stats(0)["lookups_host_ordered"] > 0
+    cache.close()

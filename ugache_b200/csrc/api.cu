@@ -1302,11 +1302,17 @@ int do_lookup(ugc_ctx* c, Replica* r, const void* keys, int key_bytes, size_t n,
                                (r->pdl & 2) != 0, s));
     p.list[kGroupHost] = r->host_sorted;
     p.host_hist = hist;
-    // CTAs for an ordered list: 40 keep 2560 rows of 256 bytes in flight, which is the window the
-    // order pays for (128- and 256-byte rows over 32 GB: 14.2 and 23.4 GB/s, with 148 CTAs 11.4 and
-    // 20.3); rows of 512 bytes fill the link from 80 CTAs on (46.9 GB/s with 40, 49.3 with 80)
-    if (r->host_ctas == r->host_ctas_default)
-      p.host_cta_cap = std::min(r->host_ctas, 40 * (int)std::max(1u, c->cfg.row_bytes / 256));
+    // CTAs for an ordered list: as many as keep 2560 rows in flight, which is the window the order pays
+    // for, and 40 at least (128- and 256-byte rows over 32 GB: 14.2 and 23.4 GB/s, with 148 CTAs 11.4
+    // and 20.3; rows of 512 bytes fill the link from 80 CTAs on: 46.9 GB/s with 40, 49.3 with 80).  Rows
+    // that move in 4-byte pieces, or in odd numbers of pieces, leave a CTA fewer at a time: 32,768 rows of
+    // 200 bytes over 1 GB with 40 / 80 CTAs 277 / 246 us, 16,384 of them over 32 GB 341 / 342; 32,768 rows
+    // of 400 bytes over 32 GB 680 / 620.
+    if (r->host_ctas == r->host_ctas_default) {
+      const int in_flight = gather_rows_in_flight(p, r->block_threads, r->vec_bytes);
+      const int want = std::max(40 * (int)std::max(1u, c->cfg.row_bytes / 256), 2560 / in_flight);
+      p.host_cta_cap = std::min(r->host_ctas, want);
+    }
     r->kernel_launches += 1;
     r->lookups_host_ordered++;
   }

@@ -2039,6 +2039,12 @@ cudaError_t launch_host_order(const uint64_t* list_host, uint64_t* sorted, const
                     host_order_shift(host_rows));
 }
 
+// Host rows a CTA of the gather has in flight: four per lane group, in pieces of 16 bytes at most.
+int gather_rows_in_flight(const GatherParams& p, int block, int vec_bytes) {
+  const int vec = std::min(16, usable_vec_bytes(p.row_bytes, vec_bytes, p.out, p.src_base, kMaxLocation));
+  return block / lanes_per_row(p.row_bytes, vec) * 4;
+}
+
 cudaError_t launch_gather_roles(const GatherParams& p_in, int grid, int block, int vec_bytes,
                                 cudaStream_t stream) {
   GatherParams p = p_in;

@@ -31,6 +31,7 @@ cudaError_t launch_lookup_group(const void* keys, int key_bytes, uint32_t n, con
                                 Counters* counters, const StreamOrder& order, int keys_per_thread, uint32_t* host_hist,
                                 uint64_t host_rows, bool pdl, cudaStream_t stream);
 
+int gather_rows_in_flight(const GatherParams& p, int block, int vec_bytes);
 cudaError_t launch_gather_roles(const GatherParams& p, int grid, int block, int vec_bytes,
                                 cudaStream_t stream);
 
