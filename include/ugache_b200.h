@@ -440,7 +440,7 @@ typedef struct {
                                      most this many rows from the host table                */
   int32_t direct_block_threads;   /* threads per CTA of the direct kernel: 128 or 256       */
   int32_t direct_tile_keys;       /* keys one warp of the direct kernel probes at a time: 8,
-                                     16 or 32; 0 = the largest that balances the warps      */
+                                     16 or 32; 0 = chosen by the batch, 1 to 32              */
   int32_t direct_deep;            /* direct kernel: 1 = twice the rows in flight per warp at
                                      3 instead of 4 CTAs per SM                             */
   int32_t direct_early_host;      /* direct kernel: the first host row of every warp's first tile

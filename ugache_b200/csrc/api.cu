@@ -1291,7 +1291,8 @@ int do_lookup(ugc_ctx* c, Replica* r, const void* keys, int key_bytes, size_t n,
   const uint64_t host_rows = c->cfg.empty_feat > 0 ? ((uint64_t)1 << c->cfg.empty_feat) : c->cfg.num_total_item;
   UGC_CUDA(launch_lookup_group(keys, key_bytes, (uint32_t)n, r->table, (uint32_t)r->id,
                                (uint32_t)c->cfg.num_device, c->cfg.empty_feat, r->list[kGroupLocal],
-                               r->list[kGroupRemote], r->list[kGroupHost], r->counters, order, r->lookup_kpt, hist, host_rows,
+                               r->list[kGroupRemote], r->list[kGroupHost], r->counters, order, r->lookup_kpt,
+                               r->sm_count, hist, host_rows,
                                (r->pdl & 1) != 0, s));
   if (prof) UGC_CUDA(cudaEventRecord(r->prof_events[r->prof_used + 1], s));
   GatherParams p = gather_params(c, r, out, (uint32_t)n);
@@ -1955,7 +1956,7 @@ int ugc_lookup_i64_static(ugc_ctx* c, int replica_id, const int64_t* keys, size_
   UGC_CUDA(cudaMemsetAsync(counters, 0, sizeof(Counters), s));
   UGC_CUDA(launch_lookup_group(keys, 8, (uint32_t)n, r->table, (uint32_t)r->id, (uint32_t)c->cfg.num_device,
                                c->cfg.empty_feat, lists, lists + kStaticMaxKeys, lists + 2 * (size_t)kStaticMaxKeys,
-                               counters, StreamOrder{}, r->lookup_kpt, nullptr, 0, false, s));
+                               counters, StreamOrder{}, r->lookup_kpt, r->sm_count, nullptr, 0, false, s));
   GatherParams p{};
   for (int i = 0; i < kMaxLocation; i++) p.src_base[i] = r->src_base[i];
   p.out = out;

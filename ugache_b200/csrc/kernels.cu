@@ -452,7 +452,7 @@ __device__ __forceinline__ void split_roles(const GatherParams& p, const uint32_
   if (cnt[kGroupLocal] == 0) {  // nothing local: the spare CTAs help the other groups
     if (cnt[kGroupRemote]) {
       n_remote = grid - n_host;
-    } else if (cnt[kGroupHost]) {
+    } else if (cnt[kGroupHost] && !p.host_hist) {
       n_host = grid;
     }
   }
@@ -898,7 +898,7 @@ __global__ void __launch_bounds__(kScatterBlock)
 // ------------------------------------------------------------------------------------
 // direct extraction: table probe and row copy in ONE kernel, no index lists
 // ------------------------------------------------------------------------------------
-// A warp owns tiles of 32 (or 16, or 8) consecutive keys -- the launcher picks the largest
+// A warp owns tiles of 32 consecutive keys or fewer, down to one (direct_tile_shift) -- the largest
 // size that leaves every warp nearly the same number of tiles; with 32-key tiles a batch of
 // 212,992 keys is 1.4 tiles per warp, so 40 % of the warps would carry twice the work of the
 // rest.  Lane l probes the table for key l of the tile;
@@ -1907,13 +1907,13 @@ inline uint32_t host_order_shift(uint64_t host_rows) {
 cudaError_t launch_lookup_group(const void* keys, int key_bytes, uint32_t n, const TableView& table,
                                 uint32_t local_loc, uint32_t host_loc, int empty_feat,
                                 uint64_t* list_local, uint64_t* list_remote, uint64_t* list_host,
-                                Counters* counters, const StreamOrder& order, int keys_per_thread, uint32_t* host_hist,
-                                uint64_t host_rows, bool pdl, cudaStream_t stream) {
+                                Counters* counters, const StreamOrder& order, int keys_per_thread, int sm_count,
+                                uint32_t* host_hist, uint64_t host_rows, bool pdl, cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
   const uint32_t mask = host_mask_of(empty_feat);
   const uint32_t shift = host_order_shift(host_rows);
   // 0: four keys a thread once that still leaves every SM four CTAs, one below
-  if (keys_per_thread == 0) keys_per_thread = n >= 148u * 4 * kBlock * 4 ? 4 : 1;
+  if (keys_per_thread == 0) keys_per_thread = n >= (uint64_t)sm_count * 4 * kBlock * 4 ? 4 : 1;
 #define UGC_LAUNCH_LOOKUP(KEYT, KPT)                                                             \
   return launch_pdl(lookup_group_kernel<KEYT, KPT>, (int)((n + kBlock * KPT - 1) / (kBlock * KPT)), \
                     kBlock, 0, stream, pdl, static_cast<const KEYT*>(keys), n, table, local_loc,   \

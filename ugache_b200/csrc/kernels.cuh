@@ -28,8 +28,8 @@ namespace ugc {
 cudaError_t launch_lookup_group(const void* keys, int key_bytes, uint32_t n, const TableView& table,
                                 uint32_t local_loc, uint32_t host_loc, int empty_feat,
                                 uint64_t* list_local, uint64_t* list_remote, uint64_t* list_host,
-                                Counters* counters, const StreamOrder& order, int keys_per_thread, uint32_t* host_hist,
-                                uint64_t host_rows, bool pdl, cudaStream_t stream);
+                                Counters* counters, const StreamOrder& order, int keys_per_thread, int sm_count,
+                                uint32_t* host_hist, uint64_t host_rows, bool pdl, cudaStream_t stream);
 
 int gather_rows_in_flight(const GatherParams& p, int block, int vec_bytes);
 cudaError_t launch_gather_roles(const GatherParams& p, int grid, int block, int vec_bytes,
