@@ -17,3 +17,14 @@ def test_rank_matches_stable_sort(built_lib, n, bits):
     ids, freqs = rt.Cache.rank_hotness(counts)
     want = np.argsort(-counts.astype(np.int64), kind="stable").astype(np.uint32)
     assert np.array_equal(ids, want) and np.array_equal(freqs, counts[want])
+
+
+def test_more_ids_than_the_library_ranks(built_lib, monkeypatch):
+    """Longer arrays go through numpy, with the same result."""
+    from ugache_b200 import runtime as rt
+    counts = np.array([3, 0, 7, 3, 7, 1], dtype=np.uint32)
+    want = rt.Cache.rank_hotness(counts)
+    monkeypatch.setattr(rt, "_RANK_MAX", 5)
+    monkeypatch.setattr(rt._lib, "lib", lambda: pytest.fail("the library refuses these"))
+    for a, b in zip(rt.Cache.rank_hotness(counts), want):
+        assert a.dtype == b.dtype and np.array_equal(a, b)

@@ -1507,7 +1507,12 @@ int ugc_placement_cost(int num_device, uint64_t N, const uint32_t* rank_ids, con
 int ugc_rank_hotness(uint64_t N, const uint32_t* counts, uint32_t* rank_ids, uint32_t* rank_freqs) {
   if (N && (!counts || !rank_ids || !rank_freqs)) return fail(UGC_ERR_INVALID, "null array");
   if (N >= 0x7fffffffull) return fail(UGC_ERR_UNSUPPORTED, "num_total_item must be below 2^31-1");
-  if (!rank_hotness(N, counts, rank_ids, rank_freqs)) return fail(UGC_ERR_NOMEM, "out of host memory");
+  bool ok = false;
+  try {
+    ok = rank_hotness(N, counts, rank_ids, rank_freqs);
+  } catch (const std::bad_alloc&) {  // no exception leaves the C interface
+  }
+  if (!ok) return fail(UGC_ERR_NOMEM, "out of host memory");
   return UGC_OK;
 }
 

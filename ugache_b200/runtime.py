@@ -16,6 +16,7 @@ POLICIES = {"intuitive": POLICY_INTUITIVE, "coll_intuitive": POLICY_INTUITIVE,
             "split_search": POLICY_SPLIT_SEARCH}
 _ELEM = {"f32": 0, "f16": 1}
 _POOL_MODE = {"sum": 0, "mean": 1}
+_RANK_MAX = 0x7ffffffe  # ids the library ranks; the placement solvers take no more either
 
 
 class PlacementArrays:
@@ -293,7 +294,7 @@ class Cache:
     @staticmethod
     def rank_hotness(counts):
         """(rank_ids, rank_freqs) for the placement solvers: ids by descending count, ties by id."""
-        if counts.dtype == np.uint32 and counts.ndim == 1:  # what hotness_read returns
+        if counts.dtype == np.uint32 and counts.ndim == 1 and len(counts) <= _RANK_MAX:  # what hotness_read returns
             counts = np.ascontiguousarray(counts)
             ids, freqs = np.empty(len(counts), np.uint32), np.empty(len(counts), np.uint32)
             check(_lib.lib().ugc_rank_hotness(len(counts), _ptr(counts), _ptr(ids), _ptr(freqs)))
