@@ -1231,7 +1231,7 @@ __global__ void __launch_bounds__(kBlock, DEEP ? 3 : 4)
 //    times the instructions; with 16-byte pieces it is 8 rows;
 //  * the loads run on over the ends of bags, and a bag's end is rare code outside the row loop.
 // Before (a lane group probed and summed bag by bag) and now: 8192 ragged bags of 26 rows of 512 bytes
-// 51 -> 22 us, 65,536 bags of 5 fp16 rows of 128 bytes 23.6 -> 15.7, 73 bags of 400 rows of 1 KiB
+// 55.7 -> 26.0 us (22 with one cache whose rows the L2 holds), 65,536 bags of 5 fp16 rows of 128 bytes 23.6 -> 15.7, 73 bags of 400 rows of 1 KiB
 // 167 -> 32, 145 bags of 877 rows of 256 bytes 108 -> 20, 186 bags of 23 rows of 128 bytes 15 -> 6.4.
 // With 16-byte pieces and many bags the rows' way through the L1 and the instructions bound it.
 template <bool F16, int VEC>
