@@ -432,7 +432,7 @@ __device__ __forceinline__ void split_roles(const GatherParams& p, const uint32_
   };
   n_host = share(t_host, cnt[kGroupHost], p.host_cta_cap);
   // an ordered host list is worked by a set number of CTAs: with more, the rows in flight spread
-  // over more of the table than the order is worth
+  // over more of the table than the order is worth (unless no row is local: then all CTAs work it)
   if (p.host_hist && cnt[kGroupHost]) n_host = max(1, min(p.host_cta_cap, ceil_div_i(cnt[kGroupHost], rmin)));
   n_remote = share(t_rem, cnt[kGroupRemote], p.remote_cta_cap);
   if (p.fixed_split) {
@@ -452,7 +452,7 @@ __device__ __forceinline__ void split_roles(const GatherParams& p, const uint32_
   if (cnt[kGroupLocal] == 0) {  // nothing local: the spare CTAs help the other groups
     if (cnt[kGroupRemote]) {
       n_remote = grid - n_host;
-    } else if (cnt[kGroupHost] && !p.host_hist) {
+    } else if (cnt[kGroupHost]) {
       n_host = grid;
     }
   }
